@@ -8,43 +8,43 @@
 // their FP64 pipe time in divisions.  Here the quotient is computed exactly
 // in 64-bit integer arithmetic instead:
 //
-//   * a, b normal: a / b = (MA / MB) * 2^(ea - eb) with 53-bit integer
-//     mantissas MA, MB.  With d = MB * 2^11 (top bit set) and
-//     U = MA * 2^63 (MA >= MB) or MA * 2^64 (MA < MB), the 53-bit quotient
-//     mantissa is Q = floor(U / d) and the remainder R = U - Q d.
-//   * Q is estimated with a 64-bit fixed-point reciprocal 2^64 + v of d
-//     (v ~ 2^128 / d - 2^64): seeded by the FP32 reciprocal of d's top 24
-//     bits and refined by two Newton-Raphson steps X' = X + X (2^128 - X d)
-//     / 2^128 in integer arithmetic, the method of division by invariant
-//     integers (T. Granlund, P. Montgomery, PLDI 1994; N. Moller,
-//     T. Granlund, IEEE Trans. Computers 60(2), 2011).
-//   * the remainder of the estimate is formed exactly in 128 bits and the
-//     estimate corrected until 0 <= R < d, so Q is exact whatever the
-//     accuracy of the reciprocal; rounding to nearest, ties to even, then
-//     compares R with d - R (the schoolbook rule: the quotient is exact, so
-//     no rounding-error analysis is involved).
+//   * a, b normal: a / b = rho 2^k with rho = mA / mb in [1, 2), mb the 53-bit
+//     mantissa of b and mA that of a, doubled where it is below mb.
+//   * Q = floor(rho 2^53), 54 bits, is formed by schoolbook long division in
+//     two digits with a 32-bit fixed-point reciprocal y of mb (the method of
+//     division by invariant integers: T. Granlund, P. Montgomery, PLDI 1994;
+//     N. Moller, T. Granlund, IEEE Trans. Computers 60(2), 2011): y is the
+//     FP32 reciprocal of b's top 24 bits refined by one Newton step, kept
+//     below the exact value, so each digit is low by a few units at most and
+//     each remainder, formed modulo 2^64, is non-negative and fits.  One
+//     comparison of the last remainder with mb makes Q exact.
+//   * A quotient of two 53-bit integers is never halfway between two 53-bit
+//     numbers (odd 54-bit Q times mb would need more than 53 bits), so
+//     (Q + 1) >> 1 is the quotient rounded to nearest.
+//
+// Bounds (y below by at most 1.5 2^-30, first digit low by less than 6 units,
+// second by less than 2) hold for any seed within the documented error of
+// rcp.approx (1 ulp).  A division is about 55 instructions; the earlier form,
+// with a 64-bit reciprocal and 128-bit remainders, was about 170 and left the
+// ALU pipe nearly as busy as the FP64 pipe.
 //
 // Results are therefore the IEEE round-to-nearest quotients, bit for bit.
 // Operands outside the fast path (zero, subnormal, infinite or NaN divisor,
 // subnormal, infinite or NaN dividend, a quotient outside the normal range)
 // take the ordinary division, which gives the IEEE result for them too.
 //
-// A divisor used with several dividends is prepared once (den_prep) and each
-// quotient then costs one 64x64 high product, one 128-bit product and a few
-// integer operations (quot).
+// A divisor used with several dividends is prepared once (den_prep); each
+// quotient then costs the two digits (quot).
 //
 // The same file holds the integer forms of the correctly rounded products by
 // constants (small integers, powers of two, literals such as 1/6) and of the
 // density guard r + 1e-30; they are described beside their code.
 //
-// The square root follows the same pattern: for normal x > 0 with 53-bit
-// mantissa MX and unbiased exponent E, N = MX * 2^(52 + (E & 1)) lies in
-// [2^104, 2^106) and sqrt(x) = sqrt(N) * 2^(floor(E / 2) - 52).  The integer
-// square root Q = floor(sqrt(N)) is estimated from a 64-bit fixed-point
-// inverse square root (FP32 seed, two Newton-Raphson steps
-// r' = r (3 - m r^2) / 2), then made exact with the remainder N - Q^2
-// (0 <= N - Q^2 <= 2Q); sqrt(N) is never a rounding midpoint (N is an
-// integer), so it rounds up exactly when N - Q^2 > Q.
+// The square root follows the same pattern: m in [1, 4) with an even exponent
+// left over, y from the FP32 inverse square root and one Newton step, the
+// first digit m y, the second from the remainder, Q = floor(sqrt(m) 2^53)
+// made exact by one comparison of m 2^106 - Q^2 with 2 Q, and (Q + 1) >> 1
+// (the root of a 53-bit number is never a rounding midpoint).
 #pragma once
 
 #include <stdint.h>
@@ -72,98 +72,90 @@ __device__ __forceinline__ float rcp_seed_f32(float x) {
   return r;
 }
 
-// 2^64 + v approximates 2^128 / d for d in [2^63, 2^64), within a few units
-// of the last place (the exact correction of each quotient absorbs the
-// remaining error).
-__device__ __forceinline__ uint64_t recip_v(uint64_t d) {
-  const uint32_t frac = (uint32_t)(d >> 40) & 0x7FFFFFu;  // 23 bits below d's leading one
-  const uint32_t rb = __float_as_uint(rcp_seed_f32(__uint_as_float(0x3F800000u | frac)));
-  // r in (1/2, 1]: 2^65 r = 2^64 + (r's 23 fraction bits << 41); r = 1 only for d = 2^63
-  uint64_t v = rb >= 0x3F800000u ? ~0ull : (uint64_t)(rb & 0x7FFFFFu) << 41;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    // E = 2^128 - (2^64 + v) d, a small signed 128-bit number; eh = floor(E / 2^64)
-    const uint64_t plo = v * d;
-    const uint64_t phi = d + __umul64hi(v, d);
-    const int64_t eh = (int64_t)(~phi + (plo == 0 ? 1ull : 0ull));
-    const uint64_t ae = eh < 0 ? (uint64_t)(-eh) : (uint64_t)eh;
-    const uint64_t c = ae + __umul64hi(v, ae);  // (2^64 + v) |eh| / 2^64
-    if (eh < 0) {
-      v = c > v ? 0ull : v - c;
-    } else {
-      const uint64_t nv = v + c;
-      v = nv < v ? ~0ull : nv;
-    }
-  }
-  return v;
+__device__ __forceinline__ uint64_t mant53(uint64_t u) {
+  return (u & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+}
+
+// low 64 bits of q m (m < 2^53): a 32x32 wide product and a 32-bit one
+__device__ __forceinline__ uint64_t mul_lo(uint32_t q, uint64_t m) {
+  return (uint64_t)q * (uint32_t)m + ((uint64_t)(q * (uint32_t)(m >> 32)) << 32);
+}
+
+// fixed-point seed: r in [1/2, 1] as an FP32 value to r 2^32 - 3 2^9, rounded
+// to a multiple of 2^9 (r + 1 - 3 2^-23 lies in [1, 2), so its fraction bits
+// are that number)
+__device__ __forceinline__ uint32_t seed_bits(float r) {
+  return __float_as_uint(r + __uint_as_float(0x3F7FFFFAu)) << 9;
+}
+
+// The fast paths take operands whose biased exponent lies in [768, 1280),
+// 2^-255 <= |x| < 2^257: products and quotients of such operands are normal,
+// so no other exponent is checked.  exp_window(high word) is below 2^30 for
+// these and not below for any other (subnormal, infinite and NaN among them).
+__device__ __forceinline__ uint32_t exp_window(uint32_t h) { return 2u * h - (768u << 21); }
+__device__ __forceinline__ uint32_t hi_word(double x) { return (uint32_t)__double2hiint(x); }
+__device__ __forceinline__ uint32_t lo_word(double x) { return (uint32_t)__double2loint(x); }
+__device__ __forceinline__ double from_words(uint32_t h, uint32_t l) { return __hiloint2double((int)h, (int)l); }
+// sign and exponent bits; mantissa bits with the leading one.  Sign and
+// exponent fields add and subtract modulo 2^32: the sign bit as exclusive or.
+__device__ __forceinline__ uint32_t sign_exp(uint32_t h) { return h & 0xFFF00000u; }
+__device__ __forceinline__ uint32_t mant_hi(uint32_t h) { return (h & 0x000FFFFFu) | 0x00100000u; }
+
+template <typename... T>
+__device__ __forceinline__ bool in_window(T... x) {
+  return (exp_window(hi_word(x)) | ...) < (1u << 30);
 }
 
 // a prepared divisor
 struct Den {
   double b;
-  uint64_t d;     // (b's 53-bit mantissa) << 11
-  uint64_t v;     // 2^64 + v ~ 2^128 / d
-  uint64_t sign;  // b's sign bit
-  int e;          // b's biased exponent
-  bool ok;        // b normal (finite, nonzero, not subnormal)
+  uint64_t mb;  // 53-bit mantissa
+  uint32_t y;   // 2^32 2^52 / mb, low by at most 1.5 2^-30 of itself
+  uint32_t w;   // exp_window
 };
 
 __device__ __forceinline__ Den den_prep(double b) {
   Den D;
-  const uint64_t ub = (uint64_t)__double_as_longlong(b);
+  const uint32_t h = hi_word(b), l = lo_word(b);
   D.b = b;
-  D.e = (int)((ub >> 52) & 0x7FF);
-  D.ok = D.e != 0 && D.e != 0x7FF;
-  D.sign = ub & 0x8000000000000000ull;
-  D.d = ((ub & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 11;
-  D.v = recip_v(D.d);
+  D.w = exp_window(h);
+  const uint32_t mh = mant_hi(h);
+  D.mb = (uint64_t)mh << 32 | l;
+  const uint32_t bh = __funnelshift_l(l, mh, 11);  // mb 2^-52 with 31 fraction bits, truncated
+  // the top 23 fraction bits as an FP32 number in [1, 2)
+  const uint32_t y0 = seed_bits(rcp_seed_f32(__uint_as_float((bh >> 8) + 0x3F000000u)));
+  // Newton: e = 1 - y0 b in units of 2^-31, made low by 2 units so that y stays low
+  const uint32_t e = 0x7FFFFFFEu - __umulhi(y0, bh);
+  D.y = y0 + __umulhi(y0, 2u * e);
   return D;
+}
+
+// results outside the fast path: zero dividends, and the ordinary division
+static __device__ __noinline__ double quot_special(double a, double b) {
+  const uint64_t ua = (uint64_t)__double_as_longlong(a), ub = (uint64_t)__double_as_longlong(b);
+  const uint32_t eb = (uint32_t)(ub >> 52) & 0x7FFu;
+  if ((ua << 1) == 0 && eb - 1u < 0x7FEu)  // +-0 / normal
+    return __longlong_as_double((long long)((ua ^ ub) & 0x8000000000000000ull));
+  return a / b;
 }
 
 // RN(a / b) for a prepared divisor
 __device__ __forceinline__ double quot(double a, const Den &D) {
-  const uint64_t ua = (uint64_t)__double_as_longlong(a);
-  const int ea = (int)((ua >> 52) & 0x7FF);
-  const uint64_t sign = (ua & 0x8000000000000000ull) ^ D.sign;
-  const uint64_t fa = ua & 0x000FFFFFFFFFFFFFull;
-  if (ea == 0 && fa == 0 && D.ok) return __longlong_as_double((long long)sign);  // +-0 / normal
-  const uint64_t ma = fa | 0x0010000000000000ull;
-  const bool ge = (ma << 11) >= D.d;
-  const int er = ea - D.e + 1022 + (ge ? 1 : 0);
-  if (!D.ok || ea == 0 || ea == 0x7FF || er < 1 || er > 2045) return a / D.b;
-  const uint64_t u1 = ge ? ma >> 1 : ma;
-  const uint64_t u0 = ge ? ma << 63 : 0ull;
-  // estimate: the exact quotient minus 0, 1 or 2 (rarely plus one)
-  uint64_t q = u1 + __umul64hi(u1, D.v);
-  // exact remainder R = U - q d in 128 bits (rhi:rlo, two's complement)
-  const uint64_t plo = q * D.d;
-  const uint64_t phi = __umul64hi(q, D.d);
-  uint64_t rlo = u0 - plo;
-  uint64_t rhi = u1 - phi - (u0 < plo ? 1ull : 0ull);
-  if ((int64_t)rhi < 0) {
-    q -= 1;
-    const uint64_t t = rlo + D.d;
-    rhi += t < rlo ? 1ull : 0ull;
-    rlo = t;
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (rhi != 0 || rlo >= D.d) {
-      q += 1;
-      rhi -= rlo < D.d ? 1ull : 0ull;
-      rlo -= D.d;
-    }
-  }
-  if (rhi != 0 || rlo >= D.d) return a / D.b;  // estimate out of range: not expected
-  // round to nearest, ties to even: compare R with d - R
-  const uint64_t rest = D.d - rlo;
-  q += (rlo > rest || (rlo == rest && (q & 1ull))) ? 1ull : 0ull;
-  uint64_t e = (uint64_t)er;
-  if (q >> 53) {  // rounded up to 2^53
-    q >>= 1;
-    e += 1;
-  }
-  return __longlong_as_double((long long)(sign | (e << 52) | (q & 0x000FFFFFFFFFFFFFull)));
+  const uint32_t h = hi_word(a), l = lo_word(a);
+  if ((exp_window(h) | D.w) >= (1u << 30)) return quot_special(a, D.b);
+  const uint64_t ma = (uint64_t)mant_hi(h) << 32 | l;
+  const bool ge = ma >= D.mb;
+  // sign and (biased exponent - 1): the mantissa's leading bit, and a carry, add one
+  const uint32_t eb = sign_exp(h) - sign_exp(hi_word(D.b)) + (ge ? 1022u << 20 : 1021u << 20);
+  // rho = mA / mb in [1, 2); Q = floor(rho 2^53) in two digits
+  const uint64_t mA = ge ? ma : ma << 1;
+  const uint32_t q1 = __umulhi((uint32_t)(mA >> 22), D.y);       // rho 2^30, low by less than 6
+  const uint64_t r1 = (mA << 30) - mul_lo(q1, D.mb);             // in [0, 6 mb)
+  const uint32_t q2 = __umulhi((uint32_t)(r1 >> 24), D.y) >> 5;  // r1 2^23 / mb, low by less than 2
+  const uint64_t r2 = (r1 << 23) - mul_lo(q2, D.mb);             // in [0, 2 mb)
+  const uint32_t t = (q2 + (r2 >= D.mb ? 2u : 1u)) >> 1;         // Q's rounding bit added, dropped
+  const uint64_t m = ((uint64_t)(eb + (q1 >> 10)) << 32 | (q1 << 22)) + t;
+  return __longlong_as_double((long long)m);
 }
 
 __device__ __forceinline__ double div(double a, double b) { return quot(a, den_prep(b)); }
@@ -186,59 +178,33 @@ __device__ __forceinline__ float rsqrt_seed_f32(float x) {
   return r;
 }
 
+static __device__ __noinline__ double sqrt_special(double x) {
+  const uint64_t ux = (uint64_t)__double_as_longlong(x);
+  if ((ux << 1) == 0) return x;  // +-0
+  return ::sqrt(x);
+}
+
 // RN(sqrt(x))
 __device__ __forceinline__ double sqrt(double x) {
   const uint64_t ux = (uint64_t)__double_as_longlong(x);
-  const int ex = (int)((ux >> 52) & 0x7FF);
-  if ((ux << 1) == 0) return x;  // +-0
-  if (ex == 0 || ex == 0x7FF || (ux >> 63)) return ::sqrt(x);
-  const uint64_t mx = (ux & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-  const int E = ex - 1023;
-  const bool odd = (E & 1) != 0;
-  // N = mx * 2^(52 + odd) = n1:n0
-  const uint64_t n1 = odd ? mx >> 11 : mx >> 12;
-  const uint64_t n0 = odd ? mx << 53 : mx << 52;
-  const uint64_t m64 = (n1 << 22) | (n0 >> 42);  // m = N / 2^104 in [1, 4), as m * 2^62
-  // FP32 seed of 1/sqrt(m) from m's top 24 bits t = m * 2^22 in [2^22, 2^24)
-  const uint32_t t = (uint32_t)(m64 >> 40);
-  const uint32_t lead = t >> 23;
-  const uint32_t fb = ((127u + lead) << 23) | ((lead ? t : t << 1) & 0x7FFFFFu);
-  const uint32_t rb = __float_as_uint(rsqrt_seed_f32(__uint_as_float(fb)));
-  // r in (1/2, 1]: R = r * 2^64 (r = 1 only for m = 1)
-  uint64_t R = rb >= 0x3F800000u ? ~0ull : (uint64_t)((rb & 0x7FFFFFu) | 0x800000u) << 40;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const uint64_t mr2 = __umul64hi(m64, __umul64hi(R, R));  // m r^2 * 2^62
-    R = __umul64hi(R, 3ull * (1ull << 62) - mr2) << 1;     // r (3 - m r^2) / 2
-  }
-  uint64_t q = __umul64hi(m64, R) >> 10;  // sqrt(N) = m r 2^52, off by a unit or two
-  const uint64_t plo = q * q, phi = __umul64hi(q, q);
-  uint64_t rlo = n0 - plo;
-  uint64_t rhi = n1 - phi - (n0 < plo ? 1ull : 0ull);
-  if ((int64_t)rhi < 0) {  // (q - 1)^2 = q^2 - (2q - 1)
-    const uint64_t add = 2 * q - 1;
-    q -= 1;
-    const uint64_t s = rlo + add;
-    rhi += s < rlo ? 1ull : 0ull;
-    rlo = s;
-  }
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const uint64_t s = 2 * q + 1;  // (q + 1)^2 = q^2 + 2q + 1
-    if (rhi != 0 || rlo >= s) {
-      q += 1;
-      rhi -= rlo < s ? 1ull : 0ull;
-      rlo -= s;
-    }
-  }
-  if (rhi != 0 || rlo > 2 * q) return ::sqrt(x);  // estimate out of range: not expected
-  q += rlo > q ? 1ull : 0ull;
-  uint64_t e = (uint64_t)((E >> 1) + 1023);
-  if (q >> 53) {
-    q >>= 1;
-    e += 1;
-  }
-  return __longlong_as_double((long long)((e << 52) | (q & 0x000FFFFFFFFFFFFFull)));
+  const uint32_t ex = (uint32_t)(ux >> 52);
+  if (ex - 1u >= 0x7FEu) return sqrt_special(x);  // zero, subnormal, infinite, NaN, negative
+  const uint32_t odd = (ex & 1u) ^ 1u;            // parity of ex - 1023
+  const uint64_t m = mant53(ux) << odd;           // m 2^-52 in [1, 4)
+  const uint32_t mh = (uint32_t)(m >> 22);        // with 30 fraction bits, truncated
+  const uint32_t y0 = seed_bits(
+      rsqrt_seed_f32(__uint_as_float(((127u + odd) << 23) | ((uint32_t)(ux >> 29) & 0x7FFFFFu))));
+  // Newton: e = 1 - m y0^2 in units of 2^-30, made low by 3 units; y = 2^32 / sqrt(m), low by at most 2^-29.3 of itself
+  const uint32_t e = 0x3FFFFFFDu - __umulhi(mh, __umulhi(y0, y0));
+  const uint32_t y = y0 + __umulhi(y0, 2u * e);
+  const uint32_t s1 = __umulhi(mh, y);                        // sqrt(m) 2^30, low by less than 7
+  const uint64_t r1 = (m << 8) - (uint64_t)s1 * s1;           // m 2^60 - s1^2 < 2^35
+  const uint32_t q2 = __umulhi((uint32_t)(r1 >> 3), y) >> 5;  // (sqrt(m) 2^30 - s1) 2^23, low by less than 2
+  const uint64_t Q = ((uint64_t)s1 << 23) + q2;
+  const uint64_t r2 = (r1 << 46) - (((uint64_t)s1 * q2) << 24) - (uint64_t)q2 * q2;  // m 2^106 - Q^2
+  const uint32_t t = (q2 + (r2 > 2 * Q ? 2u : 1u)) >> 1;
+  const uint64_t hi = (uint64_t)((ex + 1u - odd + 1021u) >> 1) << 52;
+  return __longlong_as_double((long long)(hi + ((uint64_t)s1 << 22) + t));
 }
 
 // Out-of-line forms for kernels where code size and compile time matter more
@@ -269,92 +235,142 @@ __device__ __forceinline__ Quot4 div4_call(double a0, double a1, double a2, doub
 // instruction's cost on GB300, so they leave the FP64 pipe to the products
 // and sums of two variables:
 //   * RN(K x), K a small integer: the 53-bit mantissa times K fits 57 bits;
-//     it is shifted back to 53 bits with round to nearest, ties to even
-//     (adding half a unit minus one, plus the kept part's last bit, before
-//     the shift), and a carry into bit 53 moves into the exponent field by
-//     adding the mantissa (implicit bit included) to the exponent minus one;
+//     it is shifted back to 53 bits with round to nearest, ties to even, and
+//     a carry into bit 53 moves into the exponent field by adding the
+//     mantissa (implicit bit included) to the exponent minus one;
+//   * RN(x y): the 106-bit product of the mantissas from four 32-bit products,
+//     rounded in the same way;
 //   * x * 2^-S is exact while the result stays normal: S is subtracted from
 //     the exponent field;
 //   * RN(r + 1e-30) = r whenever 1e-30 is below half a unit in the last place
 //     of r: for |r| >= 2^-44 the nearest neighbour of r lies at least 2^-97
 //     (about 6.3e-30) away on either side.
-// Operands outside these fast paths (zeros aside: zero, subnormal, huge,
-// infinite or NaN) take the ordinary FP64 operation out of line, so every
-// result is the IEEE one bit for bit.
-static __device__ __noinline__ double mul_call(double a, double b) { return a * b; }
+// Operands outside these fast paths (zero, tiny, huge, infinite or NaN) take
+// the ordinary FP64 operation, so every result is the IEEE one bit for bit.
+// Executed instructions, measured on loops of one operation: division 68
+// (a call included), root 66, product 37, square 36, product by a constant
+// 33, by a small integer 29, x / 2 11, guard 6; about 6 fewer each without
+// the check of their operands.  (Earlier forms: division 170, product by a
+// small integer 43, x / 2 15, guard 9.)  An FP64 instruction takes the time
+// of 64 issue slots.
+// (out of line: in place, the compiler executes them ahead of the branch, on the pipe that is to be spared)
+static __device__ __noinline__ double mul_call(double a, double b) {
+  // zero times finite, as in fields at rest
+  const uint32_t ah = hi_word(a), bh = hi_word(b);
+  if (((ah << 1 | lo_word(a)) == 0 || (bh << 1 | lo_word(b)) == 0) && (ah & 0x7FF00000u) != 0x7FF00000u &&
+      (bh & 0x7FF00000u) != 0x7FF00000u)
+    return from_words((ah ^ bh) & 0x80000000u, 0u);
+  return a * b;
+}
 static __device__ __noinline__ double add_call(double a, double b) { return a + b; }
 
-// RN(K x) for an integer constant 2 < K < 16 that is not a power of two
+// The product of two 53-bit mantissas xh:xl, yh:yl, P in [2^104, 2^106), as
+// 32-bit words (four 32 x 32-bit products; the middle sum fits 64 bits)
+struct Prod {
+  uint32_t w3, w2, w1, w0;
+};
+__device__ __forceinline__ Prod mant_product(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl) {
+  const uint64_t p = (uint64_t)xl * yl;
+  const uint64_t t = (uint64_t)xl * yh + (uint64_t)xh * yl + (p >> 32);
+  const uint64_t h = (uint64_t)xh * yh + (t >> 32);
+  return {(uint32_t)(h >> 32), (uint32_t)h, (uint32_t)t, (uint32_t)p};
+}
+
+// A product's bits: the top 53 bits of P (shifted down by 52, or 53 where
+// P >= 2^105), rounded by the bits below, ties to even where TIES (they can
+// occur).  eb: sign and exponent field sum less the bias and one.
+template <bool TIES>
+__device__ __forceinline__ double round_product(const Prod &p, uint32_t eb) {
+  const uint32_t top = p.w3 >> 9, s = 20u + top;
+  const uint32_t m1 = __funnelshift_r(p.w2, p.w3, s), m0 = __funnelshift_r(p.w1, p.w2, s);
+  const uint32_t w = __funnelshift_r(p.w0, p.w1, s);
+  uint32_t up = w >> 31;
+  if (TIES && w == 0x80000000u && p.w0 == 0) up = m0 & 1u;
+  const uint64_t m = ((uint64_t)(m1 + eb + (top << 20)) << 32 | m0) + up;
+  return __longlong_as_double((long long)m);
+}
+
+// RN(x c) for a positive constant c (a literal: its words fold at compile
+// time).  Where c's mantissa MC is odd, MX MC is a rounding midpoint only for
+// MX = 3 2^51 (the product needs at least 51 trailing zero bits, all of them
+// MX's), with kept part (3 MC - 1) / 2: for MC = 1 mod 4 that is odd and
+// rounding up gives the even neighbour, so no tie needs to be detected (1/6,
+// 13/12 and 2e-6 are such constants).
+__device__ __forceinline__ double mul_const_u(double x, const double c) {
+  const uint32_t h = hi_word(x), ch = hi_word(c), cl = lo_word(c);
+  const uint32_t eb = sign_exp(h) + sign_exp(ch) - (1024u << 20);
+  const Prod p = mant_product(mant_hi(h), lo_word(x), mant_hi(ch), cl);
+  return (cl & 3u) == 1u ? round_product<false>(p, eb) : round_product<true>(p, eb);
+}
+
+// RN(x y)
+__device__ __forceinline__ double mul_u(double x, double y) {
+  const uint32_t h = hi_word(x), g = hi_word(y);
+  const uint32_t eb = sign_exp(h) + sign_exp(g) - (1024u << 20);
+  return round_product<true>(mant_product(mant_hi(h), lo_word(x), mant_hi(g), lo_word(y)), eb);
+}
+
+// RN(x^2)
+__device__ __forceinline__ double square_u(double x) {
+  const uint32_t h = hi_word(x);
+  const uint32_t eb = 2u * sign_exp(h) - (1024u << 20);
+  const uint32_t mh = mant_hi(h), l = lo_word(x);
+  return round_product<true>(mant_product(mh, l, mh, l), eb);
+}
+
+// The forms *_u do not check their operands: a caller with several products
+// checks all their operands at once (in_window), so that the products lie in
+// one basic block and overlap.  Normal operands suffice where the result is
+// normal.
+
+// RN(K x) for an integer constant 2 < K < 16 that is not a power of two: the
+// 53-bit mantissa times K fits 57 bits and is shifted back by s bits
 template <int K>
-__device__ __forceinline__ double mul_small(double x) {
+__device__ __forceinline__ double mul_small_u(double x) {
   static_assert(K > 2 && K < 16 && (K & (K - 1)) != 0, "K: a small integer that is not a power of two");
   constexpr int KB = K >= 8 ? 3 : (K >= 4 ? 2 : 1);  // floor(log2 K)
-  const uint64_t ux = (uint64_t)__double_as_longlong(x);
-  const uint32_t ex = (uint32_t)(ux >> 52) & 0x7FFu;
-  // fast path: normal x with K x (rounded) below 2^1023 * 2: ex in [1, 0x7F9]
-  if (ex - 1u >= 0x7F9u) {
-    if ((ux << 1) == 0) return x;  // K * (+-0) = +-0
-    return mul_call(x, (double)K);
-  }
+  const uint32_t h = hi_word(x);
   // P = m K in [2^(52+KB), 2^(54+KB)); s = KB or KB + 1 puts P >> s in [2^52, 2^53)
-  const uint64_t P = ((ux & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) * (uint64_t)K;
-  const int s = (P >> (53 + KB)) != 0 ? KB + 1 : KB;
-  const uint64_t q = (P + ((1ull << (s - 1)) - 1ull) + ((P >> s) & 1ull)) >> s;  // in [2^52, 2^53]
-  return __longlong_as_double(
-      (long long)((ux & 0x8000000000000000ull) + ((uint64_t)(ex + (uint32_t)s - 1u) << 52) + q));
+  const uint64_t pl = (uint64_t)lo_word(x) * K;
+  const uint32_t p0 = (uint32_t)pl, p1 = mant_hi(h) * K + (uint32_t)(pl >> 32);
+  const uint32_t s = (p1 >> (21 + KB)) + KB;
+  const uint32_t m1 = p1 >> s, m0 = __funnelshift_r(p0, p1, s);
+  // the s bits shifted out, at the top of a word, plus one where the kept part is odd
+  const uint32_t w = __funnelshift_r(0u, p0, s) + (m0 & 1u);
+  const uint64_t m = ((uint64_t)(m1 + sign_exp(h) + (s << 20) - (1u << 20)) << 32 | m0) + (w > 0x80000000u ? 1u : 0u);
+  return __longlong_as_double((long long)m);
 }
 
-// RN(x c) for a positive normal constant c (a literal: its mantissa and
-// exponent fold at compile time).  With 53-bit mantissas MX, MC, the product
-// P = MX MC lies in [2^104, 2^106); a = MX 2^11 and b = MC 2^11 give
-// hi = floor(a b / 2^64) = floor(P / 2^42) exactly, the low word a b mod 2^64
-// is zero exactly when P mod 2^42 is, so the 53 kept bits, the bits below
-// them and the sticky bit are all known: round to nearest, ties to even.
+// The same with the check of their operands
+__device__ __forceinline__ double mul(double x, double y) {
+  return in_window(x, y) ? mul_u(x, y) : mul_call(x, y);
+}
+__device__ __forceinline__ double square(double x) { return in_window(x) ? square_u(x) : mul_call(x, x); }
 __device__ __forceinline__ double mul_const(double x, const double c) {
-  const uint64_t uc = (uint64_t)__double_as_longlong(c);
-  const int ec = (int)((uc >> 52) & 0x7FF);
-  const uint64_t b = ((uc & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 11;
-  const uint64_t ux = (uint64_t)__double_as_longlong(x);
-  const int ex = (int)((ux >> 52) & 0x7FF);
-  const int er = ex + ec - 1023;  // biased exponent of the result when P < 2^105
-  // fast path: x normal and the result normal and finite: er in [1, 0x7FC]
-  if (ex == 0 || ex == 0x7FF || er < 1 || er > 0x7FC) {
-    if ((ux << 1) == 0) return x;  // +-0 * c = +-0 for c > 0
-    return mul_call(x, c);
-  }
-  const uint64_t a = ((ux & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 11;
-  const uint64_t hi = __umul64hi(a, b);  // in [2^62, 2^64)
-  const uint64_t lo = a * b;
-  const int top = (int)(hi >> 63);  // P >= 2^105
-  const int sh = 10 + top;
-  const uint64_t m = hi >> sh;                      // the 53 kept bits
-  const uint64_t rest = hi & ((1ull << sh) - 1ull);  // the bits of hi below them
-  const uint64_t half = 1ull << (sh - 1);
-  const bool up = rest > half || (rest == half && (lo != 0 || (m & 1ull)));
-  const uint64_t q = m + (up ? 1ull : 0ull);  // in [2^52, 2^53]
-  return __longlong_as_double(
-      (long long)((ux & 0x8000000000000000ull) + ((uint64_t)(er + top - 1) << 52) + q));
+  return in_window(x, c) ? mul_const_u(x, c) : mul_call(x, c);
 }
+template <int K>
+__device__ __forceinline__ double mul_small(double x) {
+  return in_window(x) ? mul_small_u<K>(x) : mul_call(x, (double)K);
+}
+// the product out of line, where code size matters more than a call
+static __device__ __noinline__ double mul_out(double x, double y) { return mul(x, y); }
 
+// x / 2, unchecked
+__device__ __forceinline__ double half_u(double x) { return from_words(hi_word(x) - (1u << 20), lo_word(x)); }
 // x * 2^-S (S = 1, 2): exact for a normal result
 template <int S>
 __device__ __forceinline__ double mul_pow2_neg(double x) {
   static_assert(S >= 1 && S <= 8, "S");
-  const uint64_t ux = (uint64_t)__double_as_longlong(x);
-  const uint32_t ex = (uint32_t)(ux >> 52) & 0x7FFu;
-  // fast path: ex in [S + 1, 0x7FE]
-  if (ex - (uint32_t)(S + 1) >= (uint32_t)(0x7FF - (S + 1))) {
-    if ((ux << 1) == 0) return x;  // +-0 * 2^-S = +-0
-    return mul_call(x, 1.0 / (double)(1 << S));
-  }
-  return __longlong_as_double((long long)(ux - ((uint64_t)S << 52)));
+  const uint32_t h = hi_word(x);
+  if (exp_window(h) >= (1u << 30)) return mul_call(x, 1.0 / (double)(1 << S));
+  return from_words(h - ((uint32_t)S << 20), lo_word(x));
 }
 
-// RN(r + 1e-30)
+// RN(r + 1e-30): r for 2^-44 <= |r| < infinity
 __device__ __forceinline__ double add_1em30(double r) {
-  const uint32_t ex = (uint32_t)((uint64_t)__double_as_longlong(r) >> 52) & 0x7FFu;
-  if (ex - 979u < 0x7FFu - 979u) return r;  // 2^-44 <= |r| < infinity
-  return add_call(r, 1.e-30);
+  if (2u * hi_word(r) - (979u << 21) >= (0x7FFu - 979u) << 21) return add_call(r, 1.e-30);
+  return r;
 }
 
 #endif  // __CUDACC__

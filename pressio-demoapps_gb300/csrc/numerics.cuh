@@ -139,6 +139,14 @@ PDA_HD double mul_c(double x, double c) {
   return c * x;
 #endif
 }
+// RN(x y) on the integer pipe, out of line
+PDA_HD double mul_ip_out(double x, double y) {
+#if defined(__CUDA_ARCH__) && !defined(PDA_FP64_PIPE_DIVSQRT)
+  return ip::mul_out(x, y);
+#else
+  return x * y;
+#endif
+}
 PDA_HD double plus_es(double r) {
 #if defined(__CUDA_ARCH__) && !defined(PDA_FP64_PIPE_DIVSQRT)
   return ip::add_1em30(r);
@@ -159,6 +167,16 @@ template <bool IP, typename T>
 PDA_HD T halfx(T x) {
   if constexpr (IP) return half_of(x);
   else return T(1. / 2.) * x;
+}
+template <bool IP>
+PDA_HD double mx(double x, double y) {
+  if constexpr (IP) return mul_ip_out(x, y);
+  else return x * y;
+}
+template <bool IP>
+PDA_HD double sqx(double x) {
+  if constexpr (IP) return mul_ip_out(x, x);
+  else return x * x;
 }
 template <bool IP>
 PDA_HD double esx(double r) {
@@ -605,23 +623,23 @@ PDA_HD void euler3_flux(double F[3], const double qL[3], const double qR[3],
   constexpr double es = 1.e-30;
   const double rL = qL[0];
   const double uL = div_rn<INL>(qL[1], esx<IP>(rL));
-  const double pL = (gamma - 1) * (qL[2] - halfx<IP>(rL) * (uL * uL));
+  const double pL = mx<IP>(gamma - 1, qL[2] - mx<IP>(halfx<IP>(rL), sqx<IP>(uL)));
   const Quot2 hl = div2_rn<INL>((qL[2] + pL), qR[0], rL);  // HL and rR / rL
   const double HL = hl.q0;
-  const double FL0 = rL * uL, FL1 = rL * uL * uL + pL, FL2 = rL * uL * HL;
+  const double FL0 = mx<IP>(rL, uL), FL1 = mx<IP>(FL0, uL) + pL, FL2 = mx<IP>(FL0, HL);
   const double rR = qR[0];
   const double uR = div_rn<INL>(qR[1], esx<IP>(rR));
-  const double pR = (gamma - 1) * (qR[2] - halfx<IP>(rR) * (uR * uR));
+  const double pR = mx<IP>(gamma - 1, qR[2] - mx<IP>(halfx<IP>(rR), sqx<IP>(uR)));
   const double HR = div_rn<INL>((qR[2] + pR), rR);
-  const double FR0 = rR * uR, FR1 = rR * uR * uR + pR, FR2 = rR * uR * HR;
+  const double FR0 = mx<IP>(rR, uR), FR1 = mx<IP>(FR0, uR) + pR, FR2 = mx<IP>(FR0, HR);
   const double RT = sqrt_rn<INL>(hl.q1);
-  const Quot2 roe = div2_rn<INL>((uL + RT * uR), (HL + RT * HR), (1. + RT));
+  const Quot2 roe = div2_rn<INL>((uL + mx<IP>(RT, uR)), (HL + mx<IP>(RT, HR)), (1. + RT));
   const double u = roe.q0, H = roe.q1;
-  const double a = sqrt_rn<INL>((gamma - 1.) * (H - halfx<IP>(u * u)));
+  const double a = sqrt_rn<INL>(mx<IP>(gamma - 1., H - halfx<IP>(sqx<IP>(u))));
   const double smax = fabs(u) + a;
-  F[0] = halfx<IP>(FL0 + FR0 + smax * (qL[0] - qR[0]));
-  F[1] = halfx<IP>(FL1 + FR1 + smax * (qL[1] - qR[1]));
-  F[2] = halfx<IP>(FL2 + FR2 + smax * (qL[2] - qR[2]));
+  F[0] = halfx<IP>(FL0 + FR0 + mx<IP>(smax, qL[0] - qR[0]));
+  F[1] = halfx<IP>(FL1 + FR1 + mx<IP>(smax, qL[1] - qR[1]));
+  F[2] = halfx<IP>(FL2 + FR2 + mx<IP>(smax, qL[2] - qR[2]));
 }
 
 template <int AXIS, bool INL = false, bool IP = false>
@@ -633,32 +651,33 @@ PDA_HD void euler4_flux(double F[4], const double qL[4], const double qR[4],
   const Quot2 vl = div2_rn<INL>(qL[1], qL[2], esx<IP>(rL));
   const double uL = vl.q0, vL = vl.q1;
   const double unL = AXIS == 0 ? uL : vL;
-  const double pL = (gamma - 1) * (qL[3] - halfx<IP>(rL) * (uL * uL + vL * vL));
+  const double pL = mx<IP>(gamma - 1, qL[3] - mx<IP>(halfx<IP>(rL), sqx<IP>(uL) + sqx<IP>(vL)));
   const Quot2 hl = div2_rn<INL>((qL[3] + pL), qR[0], rL);  // HL and rR / rL
   const double HL = hl.q0;
   double FL[4];
-  FL[0] = rL * unL;
-  FL[1] = AXIS == 0 ? rL * unL * uL + pL : rL * unL * uL;
-  FL[2] = AXIS == 1 ? rL * unL * vL + pL : rL * unL * vL;
-  FL[3] = rL * unL * HL;
+  FL[0] = mx<IP>(rL, unL);
+  FL[1] = AXIS == 0 ? mx<IP>(FL[0], uL) + pL : mx<IP>(FL[0], uL);
+  FL[2] = AXIS == 1 ? mx<IP>(FL[0], vL) + pL : mx<IP>(FL[0], vL);
+  FL[3] = mx<IP>(FL[0], HL);
   const double rR = qR[0];
   const Quot2 vr = div2_rn<INL>(qR[1], qR[2], esx<IP>(rR));
   const double uR = vr.q0, vR = vr.q1;
   const double unR = AXIS == 0 ? uR : vR;
-  const double pR = (gamma - 1) * (qR[3] - halfx<IP>(rR) * (uR * uR + vR * vR));
+  const double pR = mx<IP>(gamma - 1, qR[3] - mx<IP>(halfx<IP>(rR), sqx<IP>(uR) + sqx<IP>(vR)));
   const double HR = div_rn<INL>((qR[3] + pR), rR);
   double FR[4];
-  FR[0] = rR * unR;
-  FR[1] = AXIS == 0 ? rR * unR * uR + pR : rR * unR * uR;
-  FR[2] = AXIS == 1 ? rR * unR * vR + pR : rR * unR * vR;
-  FR[3] = rR * unR * HR;
+  FR[0] = mx<IP>(rR, unR);
+  FR[1] = AXIS == 0 ? mx<IP>(FR[0], uR) + pR : mx<IP>(FR[0], uR);
+  FR[2] = AXIS == 1 ? mx<IP>(FR[0], vR) + pR : mx<IP>(FR[0], vR);
+  FR[3] = mx<IP>(FR[0], HR);
   const double RT = sqrt_rn<INL>(hl.q1);
-  const Quot3 roe = div3_rn<INL>((uL + RT * uR), (vL + RT * vR), (HL + RT * HR), (1. + RT));
+  const Quot3 roe = div3_rn<INL>((uL + mx<IP>(RT, uR)), (vL + mx<IP>(RT, vR)), (HL + mx<IP>(RT, HR)), (1. + RT));
   const double u = roe.q0, v = roe.q1, H = roe.q2;
-  const double a = sqrt_rn<INL>((gamma - 1.) * (H - halfx<IP>(u * u + v * v)));
-  const double smax = sqrt_rn<INL>(u * u + v * v) + a;
+  const double uu = sqx<IP>(u) + sqx<IP>(v);
+  const double a = sqrt_rn<INL>(mx<IP>(gamma - 1., H - halfx<IP>(uu)));
+  const double smax = sqrt_rn<INL>(uu) + a;
 #pragma unroll
-  for (int d = 0; d < 4; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + smax * (qL[d] - qR[d]));
+  for (int d = 0; d < 4; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + mx<IP>(smax, qL[d] - qR[d]));
 }
 
 template <int AXIS, bool INL = false, bool IP = false>
@@ -670,34 +689,35 @@ PDA_HD void euler5_flux(double F[5], const double qL[5], const double qR[5],
   const Quot3 vl = div3_rn<INL>(qL[1], qL[2], qL[3], esx<IP>(rL));
   const double uL = vl.q0, vL = vl.q1, wL = vl.q2;
   const double unL = AXIS == 0 ? uL : (AXIS == 1 ? vL : wL);
-  const double pL = (gamma - 1) * (qL[4] - halfx<IP>(rL) * (uL * uL + vL * vL + wL * wL));
+  const double pL = mx<IP>(gamma - 1, qL[4] - mx<IP>(halfx<IP>(rL), sqx<IP>(uL) + sqx<IP>(vL) + sqx<IP>(wL)));
   const Quot2 hl = div2_rn<INL>((qL[4] + pL), qR[0], rL);  // HL and rR / rL
   const double HL = hl.q0;
   double FL[5];
-  FL[0] = rL * unL;
-  FL[1] = AXIS == 0 ? rL * unL * uL + pL : rL * unL * uL;
-  FL[2] = AXIS == 1 ? rL * unL * vL + pL : rL * unL * vL;
-  FL[3] = AXIS == 2 ? rL * unL * wL + pL : rL * unL * wL;
-  FL[4] = rL * unL * HL;
+  FL[0] = mx<IP>(rL, unL);
+  FL[1] = AXIS == 0 ? mx<IP>(FL[0], uL) + pL : mx<IP>(FL[0], uL);
+  FL[2] = AXIS == 1 ? mx<IP>(FL[0], vL) + pL : mx<IP>(FL[0], vL);
+  FL[3] = AXIS == 2 ? mx<IP>(FL[0], wL) + pL : mx<IP>(FL[0], wL);
+  FL[4] = mx<IP>(FL[0], HL);
   const double rR = qR[0];
   const Quot3 vr = div3_rn<INL>(qR[1], qR[2], qR[3], esx<IP>(rR));
   const double uR = vr.q0, vR = vr.q1, wR = vr.q2;
   const double unR = AXIS == 0 ? uR : (AXIS == 1 ? vR : wR);
-  const double pR = (gamma - 1) * (qR[4] - halfx<IP>(rR) * (uR * uR + vR * vR + wR * wR));
+  const double pR = mx<IP>(gamma - 1, qR[4] - mx<IP>(halfx<IP>(rR), sqx<IP>(uR) + sqx<IP>(vR) + sqx<IP>(wR)));
   const double HR = div_rn<INL>((qR[4] + pR), rR);
   double FR[5];
-  FR[0] = rR * unR;
-  FR[1] = AXIS == 0 ? rR * unR * uR + pR : rR * unR * uR;
-  FR[2] = AXIS == 1 ? rR * unR * vR + pR : rR * unR * vR;
-  FR[3] = AXIS == 2 ? rR * unR * wR + pR : rR * unR * wR;
-  FR[4] = rR * unR * HR;
+  FR[0] = mx<IP>(rR, unR);
+  FR[1] = AXIS == 0 ? mx<IP>(FR[0], uR) + pR : mx<IP>(FR[0], uR);
+  FR[2] = AXIS == 1 ? mx<IP>(FR[0], vR) + pR : mx<IP>(FR[0], vR);
+  FR[3] = AXIS == 2 ? mx<IP>(FR[0], wR) + pR : mx<IP>(FR[0], wR);
+  FR[4] = mx<IP>(FR[0], HR);
   const double RT = sqrt_rn<INL>(hl.q1);
-  const Quot4 roe = div4_rn<INL>((uL + RT * uR), (vL + RT * vR), (wL + RT * wR), (HL + RT * HR), (1. + RT));
+  const Quot4 roe = div4_rn<INL>((uL + mx<IP>(RT, uR)), (vL + mx<IP>(RT, vR)), (wL + mx<IP>(RT, wR)), (HL + mx<IP>(RT, HR)), (1. + RT));
   const double u = roe.q0, v = roe.q1, w = roe.q2, H = roe.q3;
-  const double a = sqrt_rn<INL>((gamma - 1.) * (H - halfx<IP>(u * u + v * v + w * w)));
-  const double smax = sqrt_rn<INL>(u * u + v * v + w * w) + a;
+  const double uu = sqx<IP>(u) + sqx<IP>(v) + sqx<IP>(w);
+  const double a = sqrt_rn<INL>(mx<IP>(gamma - 1., H - halfx<IP>(uu)));
+  const double smax = sqrt_rn<INL>(uu) + a;
 #pragma unroll
-  for (int d = 0; d < 5; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + smax * (qL[d] - qR[d]));
+  for (int d = 0; d < 5; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + mx<IP>(smax, qL[d] - qR[d]));
 }
 
 // Shallow-water Rusanov flux.  deviation: the reference's std::pow(h, 0.5) is
@@ -712,27 +732,27 @@ PDA_HD void swe_flux(double F[3], const double qL[3], const double qR[3],
   const Quot2 vl = div2_rn<INL>(qL[1], qL[2], esx<IP>(hL));
   const double uL = vl.q0, vL = vl.q1;
   const double unL = AXIS == 0 ? uL : vL;
-  const double pL = halfx<IP>(gravity) * hL * hL;
+  const double pL = mx<IP>(mx<IP>(halfx<IP>(gravity), hL), hL);
   double FL[3];
-  FL[0] = hL * unL;
-  FL[1] = AXIS == 0 ? hL * unL * uL + pL : hL * unL * uL;
-  FL[2] = AXIS == 1 ? hL * unL * vL + pL : hL * unL * vL;
+  FL[0] = mx<IP>(hL, unL);
+  FL[1] = AXIS == 0 ? mx<IP>(FL[0], uL) + pL : mx<IP>(FL[0], uL);
+  FL[2] = AXIS == 1 ? mx<IP>(FL[0], vL) + pL : mx<IP>(FL[0], vL);
   const double hR = qR[0];
   const Quot2 vr = div2_rn<INL>(qR[1], qR[2], esx<IP>(hR));
   const double uR = vr.q0, vR = vr.q1;
   const double unR = AXIS == 0 ? uR : vR;
-  const double pR = halfx<IP>(gravity) * hR * hR;
+  const double pR = mx<IP>(mx<IP>(halfx<IP>(gravity), hR), hR);
   double FR[3];
-  FR[0] = hR * unR;
-  FR[1] = AXIS == 0 ? hR * unR * uR + pR : hR * unR * uR;
-  FR[2] = AXIS == 1 ? hR * unR * vR + pR : hR * unR * vR;
+  FR[0] = mx<IP>(hR, unR);
+  FR[1] = AXIS == 0 ? mx<IP>(FR[0], uR) + pR : mx<IP>(FR[0], uR);
+  FR[2] = AXIS == 1 ? mx<IP>(FR[0], vR) + pR : mx<IP>(FR[0], vR);
   const double hm = halfx<IP>(hL + hR);
   const double sL = sqrt_rn<INL>(hL), sR = sqrt_rn<INL>(hR);
-  const double um = div_rn<INL>((unL * sL + unR * sR), esx<IP>(sL + sR));
-  const double sg = sqrt_rn<INL>(gravity * hm);
-  const double smax = sqrt_rn<INL>(um * um) + sqrt_rn<INL>(sg * sg);
+  const double um = div_rn<INL>((mx<IP>(unL, sL) + mx<IP>(unR, sR)), esx<IP>(sL + sR));
+  const double sg = sqrt_rn<INL>(mx<IP>(gravity, hm));
+  const double smax = sqrt_rn<INL>(sqx<IP>(um)) + sqrt_rn<INL>(sqx<IP>(sg));
 #pragma unroll
-  for (int d = 0; d < 3; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + smax * (qL[d] - qR[d]));
+  for (int d = 0; d < 3; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + mx<IP>(smax, qL[d] - qR[d]));
 }
 
 // ---------------------------------------------------------------------------

@@ -10,9 +10,19 @@
 //    reconstructions of neighbouring faces with identical expression trees
 //    (impl/weno5.hpp:112-178, impl/weno3.hpp:82-131), so they are computed
 //    once per cell into shared memory and reused;
-//  * the reference's products by small integers, 1/2, 1/4 and constants and
-//    its divisions and square roots run on the integer pipe
-//    (fp64_intpipe.cuh), bit for bit;
+//  * the reference's divisions and square roots, its products by small
+//    integers, 1/2 and constants, and the products of two variables run on
+//    the integer pipe (fp64_intpipe.cuh), bit for bit; the quarter of a
+//    square is exact and joins the following sum;
+//  * an FP64 instruction takes the FP64 pipe 64 issue slots, an integer
+//    product about 30, so the two pipes share the products until both are
+//    about equally loaded: 166 FP64 instructions per 2D Euler WENO5 face
+//    (271 with all products of two variables on the FP64 pipe), FP64 pipe
+//    74 % busy, ALU pipe 61 %, issue slots 64 %.  The operands of a group of
+//    products are checked together, which leaves one basic block in which
+//    they overlap.  1024^2: 0.40 ms per face pass (0.634 ms before; 0.58 with
+//    the faster division alone, 0.425 with the weights' products moved but
+//    checked one by one and the flux's on the FP64 pipe);
 //  * the code stays small enough for the instruction cache: the per-dof
 //    loops of the cell and face phases are not unrolled (face states kept in
 //    registers by predicated moves) and every division and square root is
@@ -41,6 +51,28 @@ __device__ __forceinline__ void set_dof(double (&v)[N], int d, double x) {
 #pragma unroll
   for (int k = 0; k < N; ++k)
     if (k == d) v[k] = x;
+}
+
+// K0 x0 and K1 x1 with one check
+template <int K0, int K1>
+__device__ __forceinline__ void mul_k_all(double x0, double x1, double &y0, double &y1) {
+  if (ip::in_window(x0, x1)) {
+    y0 = ip::mul_small_u<K0>(x0);
+    y1 = ip::mul_small_u<K1>(x1);
+  } else {
+    y0 = ip::mul_call((double)K0, x0);
+    y1 = ip::mul_call((double)K1, x1);
+  }
+}
+// one weighted candidate on the FP64 pipe: (alpha s) (P / 6)
+static __device__ __noinline__ double w5_term_call(double alpha, double s, double P) {
+  if (ip::in_window(alpha, s) && (ip::hi_word(P) << 1 | ip::lo_word(P)) == 0) return P;  // alpha, s > 0
+  return (alpha * s) * (P * (1. / 6.));
+}
+
+static __device__ __noinline__ double w3_term_call(double alpha, double s, double P) {
+  if (ip::in_window(alpha, s) && (ip::hi_word(P) << 1 | ip::lo_word(P)) == 0) return P;
+  return (alpha * s) * (P * 0.5);
 }
 
 template <int SCHEME, int LANES_ = 64> struct TileCfg;
@@ -110,17 +142,46 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
 #pragma unroll 1
       for (int d = 0; d < NDPC; ++d) {
         const double a = sU[ty][d][tx], m = sU[ty][d][tx + 1], c = sU[ty][d][tx + 2];
-        const double X = w5_curv<true>(a, m, c);
-        const double D = mul_c(X, thirteenOvtwelve) * X;
-        const double YL = w5_slopeL<true>(a, m, c);
+        double a3, c3;
+        mul_k_all<3, 3>(a, c, a3, c3);
+        const double X = w5_curv(a, m, c);
+        const double YL = fma_p2(-4., m, a) + c3;  // w5_slopeL
         const double YC = a - c;
-        const double YR = w5_slopeR<true>(a, m, c);
-        const double BL = D + quarter_of(YL) * YL;
-        const double BC = D + quarter_of(YC) * YC;
-        const double BR = D + quarter_of(YR) * YR;
-        const double dL = epsilon * epsilon + mul_c(BL, 2. * epsilon) + BL * BL;
-        const double dC = epsilon * epsilon + mul_c(BC, 2. * epsilon) + BC * BC;
-        const double dR = epsilon * epsilon + mul_c(BR, 2. * epsilon) + BR * BR;
+        const double YR = fma_p2(-4., m, a3) + c;  // w5_slopeR
+        double D, sL, sC, sR;
+        if (ip::in_window(X, YL, YC, YR)) {
+          D = ip::mul_u(ip::mul_const_u(X, thirteenOvtwelve), X);
+          sL = ip::square_u(YL);
+          sC = ip::square_u(YC);
+          sR = ip::square_u(YR);
+        } else {
+          D = ip::mul_call(ip::mul_call(thirteenOvtwelve, X), X);
+          sL = ip::mul_call(YL, YL);
+          sC = ip::mul_call(YC, YC);
+          sR = ip::mul_call(YR, YR);
+        }
+        const double BL = fma_p2(0.25, sL, D);
+        const double BC = fma_p2(0.25, sC, D);
+        const double BR = fma_p2(0.25, sR, D);
+        double eL, eC, eR;
+        if (ip::in_window(BL, BC, BR)) {
+          eL = ip::mul_const_u(BL, 2. * epsilon);
+          eC = ip::mul_const_u(BC, 2. * epsilon);
+          eR = ip::mul_const_u(BR, 2. * epsilon);
+          sL = ip::square_u(BL);
+          sC = ip::square_u(BC);
+          sR = ip::square_u(BR);
+        } else {
+          eL = ip::mul_call(BL, 2. * epsilon);
+          eC = ip::mul_call(BC, 2. * epsilon);
+          eR = ip::mul_call(BR, 2. * epsilon);
+          sL = ip::mul_call(BL, BL);
+          sC = ip::mul_call(BC, BC);
+          sR = ip::mul_call(BR, BR);
+        }
+        const double dL = epsilon * epsilon + eL + sL;
+        const double dC = epsilon * epsilon + eC + sC;
+        const double dR = epsilon * epsilon + eR + sR;
         const Quot2 aL = div2_rn(oneOvten, threeOvten, dL);
         const Quot2 aR = div2_rn(threeOvten, oneOvten, dR);
         sA[ty][d][0][tx] = aL.q0;                 // uNeg alpha0 of face c+1+1/2
@@ -137,8 +198,21 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
 #pragma unroll 1
       for (int d = 0; d < NDPC; ++d) {
         const double a = sU[ty][d][tx], c = sU[ty][d][tx + 1];
-        const double B = (a - c) * (a - c);
-        const double den = epsilon * epsilon + mul_c(B, two * epsilon) + B * B;
+        const double X = a - c;
+        double B, e, q;
+        if (ip::in_window(X)) {
+          B = ip::square_u(X);
+        } else {
+          B = ip::mul_call(X, X);
+        }
+        if (ip::in_window(B)) {
+          e = ip::mul_const_u(B, two * epsilon);
+          q = ip::square_u(B);
+        } else {
+          e = ip::mul_call(B, two * epsilon);
+          q = ip::mul_call(B, B);
+        }
+        const double den = epsilon * epsilon + e + q;
         sA[ty][d][0][tx] = div_rn(oneOvthree, den);
         sA[ty][d][1][tx] = div_rn(twoOvthree, den);
       }
@@ -157,20 +231,50 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
       // left cell i = f-1: cells i-2..i+3 = sU[tx .. tx+5]; centers i-1..i+2 = sA[.][tx .. tx+3]
       const double qim2 = sU[ty][d][tx], qim1 = sU[ty][d][tx + 1], qi = sU[ty][d][tx + 2];
       const double qip1 = sU[ty][d][tx + 3], qip2 = sU[ty][d][tx + 4], qip3 = sU[ty][d][tx + 5];
-      const double p0 = mul_c(w5_pFarL<true>(qim2, qim1, qi), oneOvsix);
-      const double p1 = mul_c(w5_pMidL<true>(qim1, qi, qip1), oneOvsix);
-      const double p2 = mul_c(w5_pMidR<true>(qi, qip1, qip2), oneOvsix);
-      const double p3 = mul_c(w5_pFarR<true>(qip1, qip2, qip3), oneOvsix);
-      {
-        const double a0 = sA[ty][d][0][tx], a1 = sA[ty][d][2][tx + 1], a2 = sA[ty][d][3][tx + 2];
-        const double s = div_rn(1., (a0 + a1 + a2));
-        set_dof(uN, d, (a0 * s) * p0 + (a1 * s) * p1 + (a2 * s) * p2);
+      double k7a, k11a, k5a, k5b, k11b, k7b;
+      if (ip::in_window(qim1, qi, qip1, qip2)) {
+        k7a = ip::mul_small_u<7>(qim1);
+        k11a = ip::mul_small_u<11>(qi);
+        k5a = ip::mul_small_u<5>(qi);
+        k5b = ip::mul_small_u<5>(qip1);
+        k11b = ip::mul_small_u<11>(qip1);
+        k7b = ip::mul_small_u<7>(qip2);
+      } else {
+        k7a = ip::mul_call(7., qim1);
+        k11a = ip::mul_call(11., qi);
+        k5a = ip::mul_call(5., qi);
+        k5b = ip::mul_call(5., qip1);
+        k11b = ip::mul_call(11., qip1);
+        k7b = ip::mul_call(7., qip2);
       }
-      {
-        const double a0 = sA[ty][d][1][tx + 1], a1 = sA[ty][d][2][tx + 2], a2 = sA[ty][d][4][tx + 3];
-        const double s = div_rn(1., (a0 + a1 + a2));
-        set_dof(uP, d, (a0 * s) * p1 + (a1 * s) * p2 + (a2 * s) * p3);
+      // 6 x the candidate polynomials: w5_pFarL, w5_pMidL, w5_pMidR, w5_pFarR
+      const double P0 = fma_p2(2., qim2, -k7a) + k11a;
+      const double P1 = fma_p2(2., qip1, -qim1 + k5a);
+      const double P2 = fma_p2(2., qi, k5b) - qip2;
+      const double P3 = fma_p2(2., qip3, k11b - k7b);
+      const double n0 = sA[ty][d][0][tx], n1 = sA[ty][d][2][tx + 1], n2 = sA[ty][d][3][tx + 2];
+      const double r0 = sA[ty][d][1][tx + 1], r1 = sA[ty][d][2][tx + 2], r2 = sA[ty][d][4][tx + 3];
+      const double sn = div_rn(1., (n0 + n1 + n2)), sp = div_rn(1., (r0 + r1 + r2));
+      double t[6];
+      if (ip::in_window(P0, P1, P2, P3, n0, n1, n2, r0, r1, r2, sn, sp)) {
+        const double p0 = ip::mul_const_u(P0, oneOvsix), p1 = ip::mul_const_u(P1, oneOvsix);
+        const double p2 = ip::mul_const_u(P2, oneOvsix), p3 = ip::mul_const_u(P3, oneOvsix);
+        t[0] = ip::mul_u(ip::mul_u(n0, sn), p0);
+        t[1] = ip::mul_u(ip::mul_u(n1, sn), p1);
+        t[2] = ip::mul_u(ip::mul_u(n2, sn), p2);
+        t[3] = ip::mul_u(ip::mul_u(r0, sp), p1);
+        t[4] = ip::mul_u(ip::mul_u(r1, sp), p2);
+        t[5] = ip::mul_u(ip::mul_u(r2, sp), p3);
+      } else {
+        t[0] = w5_term_call(n0, sn, P0);
+        t[1] = w5_term_call(n1, sn, P1);
+        t[2] = w5_term_call(n2, sn, P2);
+        t[3] = w5_term_call(r0, sp, P1);
+        t[4] = w5_term_call(r1, sp, P2);
+        t[5] = w5_term_call(r2, sp, P3);
       }
+      set_dof(uN, d, t[0] + t[1] + t[2]);
+      set_dof(uP, d, t[3] + t[4] + t[5]);
     }
   } else {
     // p0 = (-q_{i-1} + 3 q_i) / 2, p1 = (q_i + q_{i+1}) / 2, p2 = (3 q_{i+1} - q_{i+2}) / 2
@@ -179,19 +283,27 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
       // left cell i = f-1: cells i-1..i+2 = sU[tx .. tx+3]; pairs i-1, i, i+1 = sA[.][tx .. tx+2]
       const double qim1 = sU[ty][d][tx], qi = sU[ty][d][tx + 1], qip1 = sU[ty][d][tx + 2],
                    qip2 = sU[ty][d][tx + 3];
-      const double p0 = half_of(-qim1 + mul_k<3>(qi));
-      const double p1 = half_of(qi + qip1);
-      const double p2 = half_of(mul_k<3>(qip1) - qip2);
-      {
-        const double a0 = sA[ty][d][0][tx], a1 = sA[ty][d][1][tx + 1];
-        const double s = div_rn(1., (a0 + a1));
-        set_dof(uN, d, (a0 * s) * p0 + (a1 * s) * p1);
+      double k3a, k3b;
+      mul_k_all<3, 3>(qi, qip1, k3a, k3b);
+      // 2 x the candidate polynomials
+      const double P0 = -qim1 + k3a, P1 = qi + qip1, P2 = k3b - qip2;
+      const double n0 = sA[ty][d][0][tx], n1 = sA[ty][d][1][tx + 1];
+      const double r0 = n1, r1 = sA[ty][d][0][tx + 2];
+      const double sn = div_rn(1., (n0 + n1)), sp = div_rn(1., (r0 + r1));
+      double t[4];
+      if (ip::in_window(P0, P1, P2, n0, n1, r1, sn, sp)) {
+        t[0] = ip::mul_u(ip::mul_u(n0, sn), ip::half_u(P0));
+        t[1] = ip::mul_u(ip::mul_u(n1, sn), ip::half_u(P1));
+        t[2] = ip::mul_u(ip::mul_u(r0, sp), ip::half_u(P1));
+        t[3] = ip::mul_u(ip::mul_u(r1, sp), ip::half_u(P2));
+      } else {
+        t[0] = w3_term_call(n0, sn, P0);
+        t[1] = w3_term_call(n1, sn, P1);
+        t[2] = w3_term_call(r0, sp, P1);
+        t[3] = w3_term_call(r1, sp, P2);
       }
-      {
-        const double a0 = sA[ty][d][1][tx + 1], a1 = sA[ty][d][0][tx + 2];
-        const double s = div_rn(1., (a0 + a1));
-        set_dof(uP, d, (a0 * s) * p1 + (a1 * s) * p2);
-      }
+      set_dof(uN, d, t[0] + t[1]);
+      set_dof(uP, d, t[2] + t[3]);
     }
   }
   double fl[NDPC];
@@ -210,8 +322,9 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
 
 // Resident blocks per SM the register allocation must allow: 32 warps per SM,
 // or fewer where the tile's shared memory admits fewer blocks (3D: 7), so the
-// cap never forces spills that buy no occupancy.  2D Euler, 1024^2: 0.634
-// against 0.638 ms per face pass at the uncapped 68 registers.
+// cap never forces spills that buy no occupancy.  2D Euler, 1024^2, whole
+// velocity: 0.848 ms with 8 blocks of 128 threads (64 registers), 0.857 with
+// 7 (72), 0.868 with 6 (80), 0.910 with 5.
 template <int FAM, int SCHEME, int NR, int LANES>
 struct FaceTileMinBlocks {
   static constexpr int kSmemPerSM = 228 * 1024, kReservedPerBlock = 1024;

@@ -112,11 +112,12 @@ __global__ void k_check_divsqrt(int mode, uint64_t seed, long per_thread, unsign
 }
 
 // Operand sets for the comparison of the integer-pipe products by constants
-// (ip::mul_small<K>, ip::mul_pow2_neg<S>, ip::mul_const) and of
-// ip::add_1em30 with the FP64
-// pipe's operations.  mode 0: random mantissas, exponents within 2^-60..2^60;
+// (ip::mul_small<K>, ip::mul_pow2_neg<S>, ip::mul_const), of the general
+// product and square (ip::mul, ip::square, counted with the constants) and of
+// ip::add_1em30 with the FP64 pipe's operations.  mode 0: random mantissas, exponents within 2^-60..2^60;
 // 1: exponents at the edges of the fast paths (subnormal results of the
-// halvings, near-overflow products, the 2^-44 bound of the density guard)
+// halvings, near-overflow products, the 2^-44 bound of the density guard, the
+// operand window of the products)
 // and short mantissas (exact products and rounding ties); 2: mantissas
 // within 64 units of 1 and of 2 - 2^-52; 3: arbitrary bit patterns (zeros,
 // subnormals, infinities, NaNs included).
@@ -135,6 +136,7 @@ __global__ void k_check_products(int mode, uint64_t seed, long per_thread, unsig
       ux = (r1 & M) | ((uint64_t)(1023 - 60 + (int)(r2 % 121)) << 52) | (r2 & (1ull << 63));
     } else if (mode == 1) {
       static const int edges[] = {0, 1, 2, 3, 4, 0x7F5, 0x7F6, 0x7F7, 0x7F8, 0x7F9, 0x7FA, 0x7FB, 0x7FE, 0x7FF,
+                                  511, 512, 767, 768, 769, 1279, 1280, 1281, 1535, 1536,
                                   975, 976, 977, 978, 979, 980, 981, 1023};
       const int e = edges[(r2 >> 8) % (sizeof(edges) / sizeof(edges[0]))];
       const uint64_t m = (r2 & 1) ? (r1 & M & ~((1ull << 40) - 1)) : (r1 & M);
@@ -146,6 +148,20 @@ __global__ void k_check_products(int mode, uint64_t seed, long per_thread, unsig
       ux = r1;
     }
     const double x = __longlong_as_double((long long)ux);
+    // a second factor: the same exponent and sign patterns, mantissas short
+    // enough for rounding ties in half of mode 1
+    uint64_t uy = (ux & ~M) ^ ((r2 >> 20) & (1ull << 63)) | (splitmix64(st) & M);
+    uint64_t uz = ux;
+    if (mode == 1 && (r2 & 2)) {
+      uy &= ~((1ull << 26) - 1);
+      uz = (ux & ~M) | (r1 & M & ~((1ull << 25) - 1));
+    }
+    if (mode == 3) uy = r2;
+    const double y = __longlong_as_double((long long)uy), z = __longlong_as_double((long long)uz);
+    nc += !same_bits(z * y, ip::mul(z, y));
+    nc += !same_bits(x * z, ip::mul(x, z));
+    nc += !same_bits(z * z, ip::square(z));
+    nc += !same_bits(y * y, ip::square(y));
     nk += !same_bits(x * 3., ip::mul_small<3>(x));
     nk += !same_bits(x * 5., ip::mul_small<5>(x));
     nk += !same_bits(x * 7., ip::mul_small<7>(x));
