@@ -294,13 +294,12 @@ int batch_num_shapes() { return F::dim == 2 ? kNumTileShapes : 1; }
 template <int SCHEME, int AXIS>
 void struct_vj_axis(const Box &b, const MeshArgs &m, const Phys &p, const double *U, const int *rowptr,
                     double *V, double *J, cudaStream_t s) {
-  constexpr int LANES = 64;
-  using Cfg = JTileCfg<FAM, SCHEME, LANES>;
+  using Cfg = JTileCfg<FAM, SCHEME>;
   constexpr int A1 = AXIS == 0 ? 1 : 0, A2 = AXIS == 2 ? 1 : 2;
   const long lines = (long)(b.hi[A1] - b.lo[A1]) * (b.hi[A2] - b.lo[A2]);
   const int nfa = b.hi[AXIS] - b.lo[AXIS] + 1;
   dim3 grid((unsigned)lines, (unsigned)div_up(nfa, Cfg::TW));
-  k_jtile<FAM, SCHEME, AXIS, LANES><<<grid, LANES, 0, s>>>(b, m, p, U, rowptr, V, J);
+  k_jtile<FAM, SCHEME, AXIS><<<grid, dim3(Cfg::LANES, Cfg::NDPC), 0, s>>>(b, m, p, U, rowptr, V, J);
 }
 
 template <int SCHEME>

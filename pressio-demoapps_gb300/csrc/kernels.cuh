@@ -39,6 +39,16 @@ template <> struct Fam<Euler1d> {
   static PDA_HD void flux_jac_ax(T JL[9], T JR[9], const T qL[3], const T qR[3], const Phys &p, int) {
     euler3_flux_jac(JL, JR, qL, qR, (T)p.gamma);
   }
+  // the left (which = 0, with the flux) or right Jacobian times 1 / jac_scale, for the Jacobian tile kernel
+  static constexpr double jac_scale = 1.;
+  template <int AXIS, class M, class S>
+  static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
+    double JL[ndpc * ndpc], JR[ndpc * ndpc];
+    if (which == 0) flux<AXIS>(fl, qL, qR, p);
+    flux_jac<AXIS>(JL, JR, qL, qR, p);
+    for (int i = 0; i < ndpc; ++i)
+      for (int j = 0; j < ndpc; ++j) set(i, j, which == 0 ? JL[i * ndpc + j] : JR[i * ndpc + j]);
+  }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<3>;
   template <int AXIS>
@@ -65,6 +75,12 @@ template <> struct Fam<Euler2d> {
   template <typename T>
   static PDA_HD void flux_jac_ax(T JL[16], T JR[16], const T qL[4], const T qR[4], const Phys &p, int ax) {
     euler4_flux_jac_ax(JL, JR, qL, qR, (T)p.gamma, ax);
+  }
+  // the left (which = 0, with the flux) or right Jacobian times 1 / jac_scale, for the Jacobian tile kernel
+  static constexpr double jac_scale = 0.5;
+  template <int AXIS, class M, class S>
+  static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
+    euler_flux_jac2<dim, AXIS, M>(which, fl, set, qL, qR, p.gamma);
   }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<4>;
@@ -95,6 +111,12 @@ template <> struct Fam<Euler3d> {
   static PDA_HD void flux_jac_ax(T JL[25], T JR[25], const T qL[5], const T qR[5], const Phys &p, int ax) {
     euler5_flux_jac_ax(JL, JR, qL, qR, (T)p.gamma, ax);
   }
+  // the left (which = 0, with the flux) or right Jacobian times 1 / jac_scale, for the Jacobian tile kernel
+  static constexpr double jac_scale = 0.5;
+  template <int AXIS, class M, class S>
+  static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
+    euler_flux_jac2<dim, AXIS, M>(which, fl, set, qL, qR, p.gamma);
+  }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<5>;
   template <int AXIS>
@@ -123,6 +145,16 @@ template <> struct Fam<Swe2d> {
   template <typename T>
   static PDA_HD void flux_jac_ax(T JL[9], T JR[9], const T qL[3], const T qR[3], const Phys &p, int ax) {
     swe_flux_jac_ax(JL, JR, qL, qR, (T)p.gravity, ax);
+  }
+  // the left (which = 0, with the flux) or right Jacobian times 1 / jac_scale, for the Jacobian tile kernel
+  static constexpr double jac_scale = 1.;
+  template <int AXIS, class M, class S>
+  static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
+    double JL[ndpc * ndpc], JR[ndpc * ndpc];
+    if (which == 0) flux<AXIS>(fl, qL, qR, p);
+    flux_jac<AXIS>(JL, JR, qL, qR, p);
+    for (int i = 0; i < ndpc; ++i)
+      for (int j = 0; j < ndpc; ++j) set(i, j, which == 0 ? JL[i * ndpc + j] : JR[i * ndpc + j]);
   }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<3>;
@@ -212,7 +244,7 @@ PDA_HD double face_value_side(int side, const double *q) {
   }
 }
 
-template <int SCHEME, typename T>
+template <int SCHEME, class M = FpMul, typename T>
 PDA_HD void face_grad_side(int side, T &u, T g[2 * SchemeTraits<SCHEME>::h], const T *q) {
   if constexpr (SCHEME == FirstOrder) {
     u = q[side];
@@ -222,8 +254,8 @@ PDA_HD void face_grad_side(int side, T &u, T g[2 * SchemeTraits<SCHEME>::h], con
     if (side == 0) weno3_neg_grad(u, g, q[0], q[1], q[2], q[3]);
     else weno3_pos_grad(u, g, q[0], q[1], q[2], q[3]);
   } else {
-    if (side == 0) weno5_neg_grad(u, g, q[0], q[1], q[2], q[3], q[4], q[5]);
-    else weno5_pos_grad(u, g, q[0], q[1], q[2], q[3], q[4], q[5]);
+    if (side == 0) weno5_neg_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5]);
+    else weno5_pos_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5]);
   }
 }
 

@@ -325,142 +325,171 @@ PDA_HD void weno5_face(double &uNeg, double &uPos, double qim2, double qim1,
   uPos = weno5_pos(qim1, qi, qip1, qip2, qip3);
 }
 
+// How a product of two variables is formed: on the FP64 pipe, or on the
+// integer pipe by a call (the same bits; kernels with enough warps to hide
+// its longer chain).
+struct FpMul {
+  template <typename T> static PDA_HD T mul(T x, T y) { return x * y; }
+};
+struct IpMul {
+  static PDA_HD double mul(double x, double y) { return mul_ip_out(x, y); }
+};
+
+// whether x is infinite or NaN, from its bits on the device
+PDA_HD bool not_finite(double x) {
+#if defined(__CUDA_ARCH__)
+  return ((uint32_t)__double2hiint(x) & 0x7FF00000u) == 0x7FF00000u;
+#else
+  return !(x - x == 0.);
+#endif
+}
+// x^3 from x and p = x^2 (see cube)
+template <class M>
+PDA_HD double cube_of(double x, double p) {
+  const double e = fma(x, x, -p);
+  const double c = M::mul(p, x);
+  const double ce = fma(p, x, -c);
+  return c + (ce + M::mul(e, x));
+}
+template <class M>
+PDA_HD float cube_of(float x, float p) { return p * x; }
+
+// One side of the WENO5 face value u and its gradient g[0..4] with respect to
+// the side's five cells, from its three candidates: p values, smoothness
+// indicators B, linear weights na / 10, and the indicators' derivatives (the
+// nine that are not zero, impl/weno5.hpp:294-310, :385-401) in the form
+//   dB0 = {d0[0], -2 d0[1], d0[2]}, dB1 = {d1[0], -2 d1[1], d1[2]} (cells 1..3),
+//   dB2 = {d2[0], -2 d2[1], d2[2]} (cells 2..4);
+// t: the candidates' derivatives, three each.  The reference's sums run over
+// all five cells of every candidate; the terms left out here are exact zeros
+// (their factors are finite unless an indicator is not, and then its c, hence
+// cS below, and so every component is NaN, as there), and a factor of -2 is
+// exact, so it joins the next sum: 94 FP64 instructions where the full loops
+// take 124.
+template <class M, typename T>
+PDA_HD void weno5_side_grad(T &u, T *g, const T p[3], const T B[3], const T na[3], const T d0[3], const T d1[3],
+                            const T d2[3], const T t[9]) {
+  constexpr T epsilon = T(1e-6);
+  T al[3], c[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const T e = B[k] + epsilon;
+    const T s = M::mul(e, e);
+    al[k] = div_rn(na[k] / T(10.), s);
+    c[k] = div_rn(-na[k], T(5.) * cube_of<M>(e, s));
+  }
+  const T aS = div_rn(T(1.), (al[0] + al[1] + al[2]));
+  const T sr = al[2] + al[1] + al[0];
+  T cS = div_rn(-T(1.), M::mul(sr, sr));
+  if (sizeof(T) == 8 && (not_finite((double)c[0]) || not_finite((double)c[1]) || not_finite((double)c[2])))
+    cS = c[0] + c[1] + c[2] + (c[0] - c[0]) + (c[1] - c[1]) + (c[2] - c[2]);  // NaN
+  const T w0 = M::mul(al[0], aS), w1 = M::mul(al[1], aS), w2 = M::mul(al[2], aS);
+  u = M::mul(w0, p[0]) + M::mul(w1, p[1]) + M::mul(w2, p[2]);
+  // da0 = {x0, -2 x1, x2}, da1 = {y0, -2 y1, y2}, da2 = {z0, -2 z1, z2}
+  const T x0 = M::mul(c[0], d0[0]), x1 = M::mul(c[0], d0[1]), x2 = M::mul(c[0], d0[2]);
+  const T y0 = M::mul(c[1], d1[0]), y1 = M::mul(c[1], d1[1]), y2 = M::mul(c[1], d1[2]);
+  const T z0 = M::mul(c[2], d2[0]), z1 = M::mul(c[2], d2[1]), z2 = M::mul(c[2], d2[2]);
+  {
+    const T S = M::mul(cS, x0);
+    T r = M::mul(M::mul(x0, aS) + M::mul(S, al[0]), p[0]) + M::mul(t[0], w0);
+    r += M::mul(M::mul(S, al[1]), p[1]);
+    r += M::mul(M::mul(S, al[2]), p[2]);
+    g[0] = r;
+  }
+  {
+    const T S = M::mul(cS, fma_p2(-T(2.), x1, y0));
+    T r = M::mul(fma_p2(-T(2.), M::mul(x1, aS), M::mul(S, al[0])), p[0]) + M::mul(t[1], w0);
+    r += M::mul(M::mul(y0, aS) + M::mul(S, al[1]), p[1]) + M::mul(t[3], w1);
+    r += M::mul(M::mul(S, al[2]), p[2]);
+    g[1] = r;
+  }
+  {
+    const T S = M::mul(cS, fma_p2(-T(2.), y1, x2) + z0);
+    T r = M::mul(M::mul(x2, aS) + M::mul(S, al[0]), p[0]) + M::mul(t[2], w0);
+    r += M::mul(fma_p2(-T(2.), M::mul(y1, aS), M::mul(S, al[1])), p[1]) + M::mul(t[4], w1);
+    r += M::mul(M::mul(z0, aS) + M::mul(S, al[2]), p[2]) + M::mul(t[6], w2);
+    g[2] = r;
+  }
+  {
+    const T S = M::mul(cS, fma_p2(-T(2.), z1, y2));
+    T r = M::mul(M::mul(S, al[0]), p[0]);
+    r += M::mul(M::mul(y2, aS) + M::mul(S, al[1]), p[1]) + M::mul(t[5], w1);
+    r += M::mul(fma_p2(-T(2.), M::mul(z1, aS), M::mul(S, al[2])), p[2]) + M::mul(t[7], w2);
+    g[3] = r;
+  }
+  {
+    const T S = M::mul(cS, z2);
+    T r = M::mul(M::mul(S, al[0]), p[0]);
+    r += M::mul(M::mul(S, al[1]), p[1]);
+    r += M::mul(M::mul(z2, aS) + M::mul(S, al[2]), p[2]) + M::mul(t[8], w2);
+    g[4] = r;
+  }
+}
+// an outer candidate's derivatives from 13 x curvature X and slope Y: Y / 2 +
+// X / 6, -2 (Y + X / 6), 3 Y / 2 + X / 6 (RN(X / 3) is 2 RN(X / 6))
+template <typename T>
+PDA_HD void w5_outer_derivs(T &a, T &b, T &c, T X, T Y) {
+  const T D = div_const(X, T(6.), T(1.) / T(6.));
+  a = fma_p2(T(0.5), Y, D);
+  b = Y + D;
+  c = fma_p2(T(0.5), T(3.) * Y, D);
+}
+// the middle candidate's: Y / 2 + X / 6, -2 X / 6, -Y / 2 + X / 6
+template <typename T>
+PDA_HD void w5_mid_derivs(T &a, T &b, T &c, T X, T Y) {
+  const T D = div_const(X, T(6.), T(1.) / T(6.));
+  a = fma_p2(T(0.5), Y, D);
+  b = D;
+  c = fma_p2(-T(0.5), Y, D);
+}
+// smoothness indicator from curvature X and slope Y (the quarter of a square is exact)
+template <class M, typename T>
+PDA_HD T w5_indicator(T X, T Y) {
+  return fma_p2(T(1.) / T(4.), M::mul(Y, Y), T(13.) / T(12.) * M::mul(X, X));
+}
+
 // WENO5 with the gradient of the two face values with respect to the six
 // stencil values q_{i-2..i+3}: gNeg[5] == 0, gPos[0] == 0.
 // one side of weno5_face_grad: uNeg and its gradient
-template <typename T>
+template <class M = FpMul, typename T>
 PDA_HD void weno5_neg_grad(T &uNeg, T gNeg[6], T qim2, T qim1, T qi, T qip1, T qip2, T qip3) {
-  constexpr T epsilon = T(1e-6);
-  constexpr T two = T(2.), three = T(3.), four = T(4.), five = T(5.), seven = T(7.),
-                   eleven = T(11.);
-  constexpr T oneOvfour = T(1.) / T(4.), oneOvsix = T(1.) / T(6.),
-                   oneOvten = T(1.) / T(10.), threeOvten = T(3.) / T(10.),
-                   sixOvten = T(6.) / T(10.), thirteenOvtwelve = T(13.) / T(12.);
-  {
-    const T p0 = w5_pFarL(qim2, qim1, qi) * oneOvsix;
-    const T p1 = w5_pMidL(qim1, qi, qip1) * oneOvsix;
-    const T p2 = w5_pMidR(qi, qip1, qip2) * oneOvsix;
-    const T dp0[5] = {T(1.) / T(3.), -T(7.) / T(6.), T(11.) / T(6.), T(0.), T(0.)};
-    const T dp1[5] = {T(0.), -T(1.) / T(6.), T(5.) / T(6.), T(1.) / T(3.), T(0.)};
-    const T dp2[5] = {T(0.), T(0.), T(1.) / T(3.), T(5.) / T(6.), -T(1.) / T(6.)};
-    const T B0 = thirteenOvtwelve * sq(w5_curv(qim2, qim1, qi)) +
-                      oneOvfour * sq(w5_slopeL(qim2, qim1, qi));
-    const T B1 = thirteenOvtwelve * sq(w5_curv(qim1, qi, qip1)) +
-                      oneOvfour * sq(qim1 - qip1);
-    const T B2 = thirteenOvtwelve * sq(w5_curv(qi, qip1, qip2)) +
-                      oneOvfour * sq(w5_slopeR(qi, qip1, qip2));
-    // derivative terms (impl/weno5.hpp:294-310), the products by 2 and 1/2 fused
-    const T X0 = T(13.) * w5_curv(qim2, qim1, qi), Y0 = w5_slopeL(qim2, qim1, qi);
-    const T X1 = T(13.) * fma_p2(-T(2.), qi, qip1 + qim1), Y1 = qim1 - qip1;
-    const T X2 = T(13.) * w5_curv(qip2, qip1, qi), Y2 = w5_slopeL(qip2, qip1, qi);
-    T dB0[5], dB1[5], dB2[5];
-    dB0[0] = fma_p2(T(0.5), Y0, div_const(X0, T(6.), T(1.) / T(6.)));
-    dB0[1] = fma_p2(-T(2.), Y0, div_const(-X0, T(3.), T(1.) / T(3.)));
-    dB0[2] = fma_p2(T(0.5), T(3.) * Y0, div_const(X0, T(6.), T(1.) / T(6.)));
-    dB0[3] = T(0.);
-    dB0[4] = T(0.);
-    dB1[0] = T(0.);
-    dB1[1] = fma_p2(T(0.5), Y1, div_const(X1, T(6.), T(1.) / T(6.)));
-    dB1[2] = div_const(-X1, T(3.), T(1.) / T(3.));
-    dB1[3] = fma_p2(-T(0.5), Y1, div_const(X1, T(6.), T(1.) / T(6.)));
-    dB1[4] = T(0.);
-    dB2[0] = T(0.);
-    dB2[1] = T(0.);
-    dB2[2] = fma_p2(T(0.5), T(3.) * Y2, div_const(X2, T(6.), T(1.) / T(6.)));
-    dB2[3] = fma_p2(-T(2.), Y2, div_const(-X2, T(3.), T(1.) / T(3.)));
-    dB2[4] = fma_p2(T(0.5), Y2, div_const(X2, T(6.), T(1.) / T(6.)));
-    const T alpha0 = div_rn(oneOvten, sq(epsilon + B0));
-    const T alpha1 = div_rn(sixOvten, sq(epsilon + B1));
-    const T alpha2 = div_rn(threeOvten, sq(epsilon + B2));
-    const T alphaSInv = div_rn(T(1.), (alpha0 + alpha1 + alpha2));
-    const T c0 = div_rn(-T(1.), (T(5.) * cube(B0 + epsilon)));
-    const T c1 = div_rn(-T(6.), (T(5.) * cube(B1 + epsilon)));
-    const T c2 = div_rn(-T(3.), (T(5.) * cube(B2 + epsilon)));
-    const T cS = div_rn(-T(1.), sq(alpha2 + alpha1 + alpha0));
-    const T w0 = alpha0 * alphaSInv;
-    const T w1 = alpha1 * alphaSInv;
-    const T w2 = alpha2 * alphaSInv;
-    for (int i = 0; i < 5; i++) {
-      const T da0 = c0 * dB0[i];
-      const T da1 = c1 * dB1[i];
-      const T da2 = c2 * dB2[i];
-      const T daS = cS * (da0 + da1 + da2);
-      T g = add_table_prod((da0 * alphaSInv + daS * alpha0) * p0, dp0[i], w0);
-      g += add_table_prod((da1 * alphaSInv + daS * alpha1) * p1, dp1[i], w1);
-      g += add_table_prod((da2 * alphaSInv + daS * alpha2) * p2, dp2[i], w2);
-      gNeg[i] = g;
-    }
-    gNeg[5] = T(0.);
-    uNeg = w0 * p0 + w1 * p1 + w2 * p2;
-  }
+  constexpr T oneOvsix = T(1.) / T(6.);
+  const T na[3] = {T(1.), T(6.), T(3.)};
+  const T t[9] = {T(1.) / T(3.),  -T(7.) / T(6.), T(11.) / T(6.), -T(1.) / T(6.), T(5.) / T(6.),
+                  T(1.) / T(3.),  T(1.) / T(3.),  T(5.) / T(6.),  -T(1.) / T(6.)};
+  const T p[3] = {w5_pFarL(qim2, qim1, qi) * oneOvsix, w5_pMidL(qim1, qi, qip1) * oneOvsix,
+                  w5_pMidR(qi, qip1, qip2) * oneOvsix};
+  const T C0 = w5_curv(qim2, qim1, qi), Y0 = w5_slopeL(qim2, qim1, qi), Y1 = qim1 - qip1;
+  const T B[3] = {w5_indicator<M>(C0, Y0), w5_indicator<M>(w5_curv(qim1, qi, qip1), Y1),
+                  w5_indicator<M>(w5_curv(qi, qip1, qip2), w5_slopeR(qi, qip1, qip2))};
+  T d0[3], d1[3], d2[3];
+  w5_outer_derivs(d0[0], d0[1], d0[2], T(13.) * C0, Y0);
+  w5_mid_derivs(d1[0], d1[1], d1[2], T(13.) * fma_p2(-T(2.), qi, qip1 + qim1), Y1);
+  w5_outer_derivs(d2[2], d2[1], d2[0], T(13.) * w5_curv(qip2, qip1, qi), w5_slopeL(qip2, qip1, qi));
+  weno5_side_grad<M>(uNeg, gNeg, p, B, na, d0, d1, d2, t);
+  gNeg[5] = T(0.);
 }
 
 // one side of weno5_face_grad: uPos and its gradient
-template <typename T>
+template <class M = FpMul, typename T>
 PDA_HD void weno5_pos_grad(T &uPos, T gPos[6], T qim2, T qim1, T qi, T qip1, T qip2, T qip3) {
-  constexpr T epsilon = T(1e-6);
-  constexpr T two = T(2.), three = T(3.), four = T(4.), five = T(5.), seven = T(7.),
-                   eleven = T(11.);
-  constexpr T oneOvfour = T(1.) / T(4.), oneOvsix = T(1.) / T(6.),
-                   oneOvten = T(1.) / T(10.), threeOvten = T(3.) / T(10.),
-                   sixOvten = T(6.) / T(10.), thirteenOvtwelve = T(13.) / T(12.);
-  {
-    const T p0 = w5_pMidL(qim1, qi, qip1) * oneOvsix;
-    const T p1 = w5_pMidR(qi, qip1, qip2) * oneOvsix;
-    const T p2 = w5_pFarR(qip1, qip2, qip3) * oneOvsix;
-    const T dp0[5] = {-T(1.) / T(6.), T(5.) / T(6.), T(1.) / T(3.), T(0.), T(0.)};
-    const T dp1[5] = {T(0.), T(1.) / T(3.), T(5.) / T(6.), -T(1.) / T(6.), T(0.)};
-    const T dp2[5] = {T(0.), T(0.), T(11.) / T(6.), -T(7.) / T(6.), T(1.) / T(3.)};
-    const T B0 = thirteenOvtwelve * sq(w5_curv(qim1, qi, qip1)) +
-                      oneOvfour * sq(w5_slopeL(qim1, qi, qip1));
-    const T B1 = thirteenOvtwelve * sq(w5_curv(qi, qip1, qip2)) +
-                      oneOvfour * sq(qi - qip2);
-    const T B2 = thirteenOvtwelve * sq(w5_curv(qip1, qip2, qip3)) +
-                      oneOvfour * sq(w5_slopeR(qip1, qip2, qip3));
-    // derivative terms (impl/weno5.hpp:385-401), the products by 2, 4 and 1/2 fused
-    const T X0 = T(13.) * fma_p2(-T(2.), qi, qip1 + qim1), Y0 = fma_p2(-T(4.), qi, T(3.) * qip1 + qim1);
-    const T X1 = T(13.) * w5_curv(qip2, qip1, qi), Y1 = qi - qip2;
-    const T X2 = T(13.) * w5_curv(qip3, qip2, qip1), Y2 = w5_slopeL(qip3, qip2, qip1);
-    T dB0[5], dB1[5], dB2[5];
-    dB0[0] = fma_p2(T(0.5), Y0, div_const(X0, T(6.), T(1.) / T(6.)));
-    dB0[1] = fma_p2(-T(2.), Y0, -div_const(X0, T(3.), T(1.) / T(3.)));
-    dB0[2] = fma_p2(T(0.5), T(3.) * Y0, div_const(X0, T(6.), T(1.) / T(6.)));
-    dB0[3] = T(0.);
-    dB0[4] = T(0.);
-    dB1[0] = T(0.);
-    dB1[1] = fma_p2(T(0.5), Y1, div_const(X1, T(6.), T(1.) / T(6.)));
-    dB1[2] = div_const(-X1, T(3.), T(1.) / T(3.));
-    dB1[3] = fma_p2(-T(0.5), Y1, div_const(X1, T(6.), T(1.) / T(6.)));
-    dB1[4] = T(0.);
-    dB2[0] = T(0.);
-    dB2[1] = T(0.);
-    dB2[2] = fma_p2(T(0.5), T(3.) * Y2, div_const(X2, T(6.), T(1.) / T(6.)));
-    dB2[3] = fma_p2(-T(2.), Y2, div_const(-X2, T(3.), T(1.) / T(3.)));
-    dB2[4] = fma_p2(T(0.5), Y2, div_const(X2, T(6.), T(1.) / T(6.)));
-    const T alpha0 = div_rn(threeOvten, sq(epsilon + B0));
-    const T alpha1 = div_rn(sixOvten, sq(epsilon + B1));
-    const T alpha2 = div_rn(oneOvten, sq(epsilon + B2));
-    const T alphaSInv = div_rn(T(1.), (alpha0 + alpha1 + alpha2));
-    const T c0 = div_rn(-T(3.), (T(5.) * cube(B0 + epsilon)));
-    const T c1 = div_rn(-T(6.), (T(5.) * cube(B1 + epsilon)));
-    const T c2 = div_rn(-T(1.), (T(5.) * cube(B2 + epsilon)));
-    const T cS = div_rn(-T(1.), sq(alpha2 + alpha1 + alpha0));
-    const T w0 = alpha0 * alphaSInv;
-    const T w1 = alpha1 * alphaSInv;
-    const T w2 = alpha2 * alphaSInv;
-    for (int i = 0; i < 5; i++) {
-      const T da0 = c0 * dB0[i];
-      const T da1 = c1 * dB1[i];
-      const T da2 = c2 * dB2[i];
-      const T daS = cS * (da0 + da1 + da2);
-      T g = add_table_prod((da0 * alphaSInv + daS * alpha0) * p0, dp0[i], w0);
-      g += add_table_prod((da1 * alphaSInv + daS * alpha1) * p1, dp1[i], w1);
-      g += add_table_prod((da2 * alphaSInv + daS * alpha2) * p2, dp2[i], w2);
-      gPos[i + 1] = g;
-    }
-    gPos[0] = T(0.);
-    uPos = w0 * p0 + w1 * p1 + w2 * p2;
-  }
+  constexpr T oneOvsix = T(1.) / T(6.);
+  const T na[3] = {T(3.), T(6.), T(1.)};
+  const T t[9] = {-T(1.) / T(6.), T(5.) / T(6.),  T(1.) / T(3.),  T(1.) / T(3.), T(5.) / T(6.),
+                  -T(1.) / T(6.), T(11.) / T(6.), -T(7.) / T(6.), T(1.) / T(3.)};
+  const T p[3] = {w5_pMidL(qim1, qi, qip1) * oneOvsix, w5_pMidR(qi, qip1, qip2) * oneOvsix,
+                  w5_pFarR(qip1, qip2, qip3) * oneOvsix};
+  const T Y1 = qi - qip2;
+  const T B[3] = {w5_indicator<M>(w5_curv(qim1, qi, qip1), w5_slopeL(qim1, qi, qip1)),
+                  w5_indicator<M>(w5_curv(qi, qip1, qip2), Y1),
+                  w5_indicator<M>(w5_curv(qip1, qip2, qip3), w5_slopeR(qip1, qip2, qip3))};
+  T d0[3], d1[3], d2[3];
+  w5_outer_derivs(d0[0], d0[1], d0[2], T(13.) * fma_p2(-T(2.), qi, qip1 + qim1),
+                  fma_p2(-T(4.), qi, T(3.) * qip1 + qim1));
+  w5_mid_derivs(d1[0], d1[1], d1[2], T(13.) * w5_curv(qip2, qip1, qi), Y1);
+  w5_outer_derivs(d2[2], d2[1], d2[0], T(13.) * w5_curv(qip3, qip2, qip1), w5_slopeL(qip3, qip2, qip1));
+  weno5_side_grad<M>(uPos, gPos + 1, p, B, na, d0, d1, d2, t);
+  gPos[0] = T(0.);
 }
 
 PDA_HD void weno5_face_grad(double &uNeg, double &uPos, double gNeg[6],
@@ -1156,6 +1185,130 @@ template <int AXIS, typename T>
 PDA_HD void euler5_flux_jac(T JL[25], T JR[25], const T qL[5],
                             const T qR[5], T gamma) {
   euler5_flux_jac_ax(JL, JR, qL, qR, gamma, AXIS);
+}
+
+// The 2D (DIM = 2) or 3D Euler face's Rusanov flux fl and twice its two
+// Jacobians, J2L = 2 dF/dqL and J2R = 2 dF/dqR, for a normal along a fixed
+// axis: euler4/5_flux and euler4/5_flux_jac with the products by the normal's
+// zeros and ones left out, what the three have in common formed once, and the
+// factors of 1/2 (exact) joined to a sum or left to the caller, who scales by
+// half as much; every other rounding is theirs.  One call forms one of the
+// two (side 0: J2L and the flux, side 1: J2R), so that two warps share a
+// face's work; set(row, column, x) receives the entries.
+template <int DIM, int AXIS, class M, class S>
+PDA_HD void euler_flux_jac2(int which, double *fl, S set, const double *qL, const double *qR, double gamma) {
+  constexpr int N = DIM + 2, E = DIM + 1;
+  constexpr double es = 1.e-30;
+  const double gm1 = gamma - 1.;
+  struct Side {
+    double v[DIM], V2, p, H;  // velocities, |v|^2, pressure, enthalpy
+  };
+  auto side = [&](Side &o, const double *q) {
+    const double r = q[0];
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) o.v[k] = div_rn(q[1 + k], (r + es));
+    o.V2 = M::mul(o.v[0], o.v[0]);
+#pragma unroll
+    for (int k = 1; k < DIM; ++k) o.V2 = o.V2 + M::mul(o.v[k], o.v[k]);
+    o.p = M::mul(gm1, fma_p2(-0.5, M::mul(r, o.V2), q[E]));
+    o.H = div_rn(q[E] + o.p, r);
+  };
+  Side L, R;
+  side(L, qL);
+  side(R, qR);
+  const double rL = qL[0], rR = qR[0];
+  const double r = sqrt_rn(M::mul(rR, rL));
+  const double RT = sqrt_rn(div_rn(rR, rL));
+  const double T1 = 1. + RT;
+  double v[DIM];
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) v[k] = div_rn(L.v[k] + M::mul(RT, R.v[k]), T1);
+  const double H = div_rn(L.H + M::mul(RT, R.H), T1);
+  double V2 = M::mul(v[0], v[0]);
+#pragma unroll
+  for (int k = 1; k < DIM; ++k) V2 = V2 + M::mul(v[k], v[k]);
+  const double a = sqrt_rn(M::mul(gm1, fma_p2(-0.5, V2, H)));
+  const double smax = sqrt_rn(V2) + a;
+  const double V2es = V2 + es;
+  const double sv = sqrt_rn(V2es);
+  double rel[DIM];
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) rel[k] = div_rn(v[k], sv);
+  const double ga = div_rn(0.5 * gm1, a);
+  double dq[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) dq[k] = qL[k] - qR[k];
+  if (which == 0) {
+    const double mL = M::mul(rL, L.v[AXIS]), mR = M::mul(rR, R.v[AXIS]);
+    fl[0] = 0.5 * (mL + mR + M::mul(smax, dq[0]));
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      double fL = M::mul(mL, L.v[k]), fR = M::mul(mR, R.v[k]);
+      if (k == AXIS) {
+        fL = fL + L.p;
+        fR = fR + R.p;
+      }
+      fl[1 + k] = 0.5 * (fL + fR + M::mul(smax, dq[1 + k]));
+    }
+    fl[E] = 0.5 * (M::mul(mL, L.H) + M::mul(mR, R.H) + M::mul(smax, dq[E]));
+  }
+  Side X;
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) X.v[k] = which == 0 ? L.v[k] : R.v[k];
+  X.V2 = which == 0 ? L.V2 : R.V2;
+  X.H = which == 0 ? L.H : R.H;
+  const double aX = sqrt_rn(M::mul(gm1, fma_p2(-0.5, X.V2, X.H)));
+  const double rX = which == 0 ? rL : rR, diag = which == 0 ? smax : -smax;
+  const double inv = div_rn(1., rX + r);
+  double g[N];
+  double m = M::mul(X.v[0] + v[0], rel[0]), VV = M::mul(X.v[0], v[0]);
+#pragma unroll
+  for (int k = 1; k < DIM; ++k) {
+    m = m + M::mul(X.v[k] + v[k], rel[k]);
+    VV = VV + M::mul(X.v[k], v[k]);
+  }
+  const double t = fma_p2(0.5, M::mul(gamma - 2., X.V2),
+                          fma_p2(0.5, (V2es + VV) + (X.H - H), -div_rn(M::mul(aX, aX), gm1)));
+  g[0] = M::mul(inv, fma_p2(-0.5, m, M::mul(ga, t)));
+#pragma unroll
+  for (int k = 0; k < DIM; ++k)
+    g[1 + k] = M::mul(inv, fma_p2(-0.5, div_rn(M::mul(gm1, v[k] + M::mul(gm1, X.v[k])), a), rel[k]));
+  g[E] = 0.5 * div_rn(M::mul(M::mul(inv, gamma), gm1), a);
+  const double un = X.v[AXIS], gV2 = M::mul(gm1, X.V2);
+  double w[DIM];  // gm1 v
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) w[k] = M::mul(gm1, X.v[k]);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const double tt = M::mul(g[j], dq[i]);
+      bool zero = false;
+      double e = 0.;
+      if (i == 0) {
+        if (j == 1 + AXIS) e = 1.;
+        else zero = true;
+      } else if (i < E) {
+        const int k = i - 1, l = j - 1;
+        if (j == 0) e = k == AXIS ? fma_p2(0.5, gV2, -M::mul(X.v[k], un)) : -M::mul(X.v[k], un);
+        else if (j == E) {
+          if (k == AXIS) e = gm1;
+          else zero = true;
+        } else if (k == AXIS) e = l == AXIS ? X.v[k] - w[k] + un : -w[l];
+        else if (l == AXIS) e = X.v[k];
+        else if (l == k) e = un;
+        else zero = true;
+      } else {
+        if (j == 0) e = M::mul(fma_p2(0.5, gV2, -X.H), un);
+        else if (j == E) e = M::mul(gamma, un);
+        else e = j - 1 == AXIS ? X.H - M::mul(w[j - 1], un) : -M::mul(w[j - 1], un);
+      }
+      if (i == j) {
+        e = zero ? diag : diag + e;
+        zero = false;
+      }
+      set(i, j, zero ? tt : e + tt);
+    }
 }
 
 // Shallow-water Rusanov flux Jacobian (generic normal).  deviation: pow(x,0.5)
