@@ -688,6 +688,23 @@ void check_launch(pda_problem &P, int n = 1) {
   PDA_CUDA(cudaGetLastError());
 }
 
+// the side stream, behind what the problem's stream has been given; its work
+// is joined before the call returns
+cudaStream_t fork_side(pda_problem &P) {
+  if (!P.side) {
+    PDA_CUDA(cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking));
+    PDA_CUDA(cudaEventCreateWithFlags(&P.evFork, cudaEventDisableTiming));
+    PDA_CUDA(cudaEventCreateWithFlags(&P.evJoin, cudaEventDisableTiming));
+  }
+  PDA_CUDA(cudaEventRecord(P.evFork, P.stream));
+  PDA_CUDA(cudaStreamWaitEvent(P.side, P.evFork, 0));
+  return P.side;
+}
+void join_side(pda_problem &P) {
+  PDA_CUDA(cudaEventRecord(P.evJoin, P.side));
+  PDA_CUDA(cudaStreamWaitEvent(P.stream, P.evJoin, 0));
+}
+
 // --------------------------------------------------------------- evaluation
 void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t *ev = nullptr) {
   check_evaluable(P);
@@ -711,18 +728,11 @@ void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t 
       // (1024^2 Riemann WENO5: 1.302 ms per velocity against 1.319 ms with
       // the passes in sequence).  The profiling path (ev) keeps the
       // sequence, one pass at a time.
-      if (!P.side) {
-        PDA_CUDA(cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking));
-        PDA_CUDA(cudaEventCreateWithFlags(&P.evFork, cudaEventDisableTiming));
-        PDA_CUDA(cudaEventCreateWithFlags(&P.evJoin, cudaEventDisableTiming));
-      }
-      PDA_CUDA(cudaEventRecord(P.evFork, P.stream));
-      PDA_CUDA(cudaStreamWaitEvent(P.side, P.evFork, 0));
+      fork_side(P);
       P.L->struct_faces(P.scheme, 0, b, P.phys, U, Fb[0], P.stream);
       P.L->struct_faces(P.scheme, 1, b, P.phys, U, Fb[1], P.side);
       if (P.dim == 3) P.L->struct_faces(P.scheme, 2, b, P.phys, U, Fb[2], P.stream);
-      PDA_CUDA(cudaEventRecord(P.evJoin, P.side));
-      PDA_CUDA(cudaStreamWaitEvent(P.stream, P.evJoin, 0));
+      join_side(P);
       const double *Fc[3] = {Fb[0], Fb[1], Fb[2]};
       P.L->struct_balance(b, ma, P.phys, U, Fc, V, P.stream);
       check_launch(P, P.dim + 1);
@@ -757,13 +767,18 @@ void velocity_and_jacobian(pda_problem &P, const double *U, double *V, double *J
     build_near_table(P, true);
     pattern_to_device(P);
     P.nearT.sync();
+    // near-boundary rows beside the inner ones (disjoint rows of V and J), on
+    // the side stream: their one launch is a chain of latencies
+    const bool near = P.nearT.t.nrows > 0;
+    cudaStream_t ns = near ? fork_side(P) : P.stream;
+    if (near) {
+      P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, ns);
+      check_launch(P);
+    }
     int nl = 0;
     P.L->struct_vj(P.scheme, P.jbox, ma, P.phys, U, P.d_rowptr.p, V, J, P.stream, &nl);
     check_launch(P, nl);
-    if (P.nearT.t.nrows > 0) {
-      P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, P.stream);
-      check_launch(P);
-    }
+    if (near) join_side(P);
     return;
   }
   build_inner_table(P, true);
@@ -776,14 +791,7 @@ void velocity_and_jacobian(pda_problem &P, const double *U, double *V, double *J
   if (both) {
     // the two row sets are independent (disjoint rows of V and J): fork the
     // near-boundary rows onto a second stream and join before returning
-    if (!P.side) {
-      PDA_CUDA(cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking));
-      PDA_CUDA(cudaEventCreateWithFlags(&P.evFork, cudaEventDisableTiming));
-      PDA_CUDA(cudaEventCreateWithFlags(&P.evJoin, cudaEventDisableTiming));
-    }
-    PDA_CUDA(cudaEventRecord(P.evFork, P.stream));
-    PDA_CUDA(cudaStreamWaitEvent(P.side, P.evFork, 0));
-    ns = P.side;
+    ns = fork_side(P);
   }
   if (P.nearT.t.nrows > 0) {
     P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, ns);
@@ -793,10 +801,7 @@ void velocity_and_jacobian(pda_problem &P, const double *U, double *V, double *J
     P.L->rows_vj_inner(P.scheme, P.innerT.t, ma, P.phys, U, P.d_rowptr.p, V, J, P.stream);
     check_launch(P);
   }
-  if (both) {
-    PDA_CUDA(cudaEventRecord(P.evJoin, P.side));
-    PDA_CUDA(cudaStreamWaitEvent(P.stream, P.evJoin, 0));
-  }
+  if (both) join_side(P);
 }
 
 // ------------------------------------------------------------------ create
