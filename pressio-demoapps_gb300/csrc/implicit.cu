@@ -12,205 +12,339 @@
 // solve J_R d = R, stop before updating when |d|_2 < tol (Pressio's default
 // criterion, the absolute l2 norm of the correction), else y <- y - d.
 // BiCGSTAB follows the standard preconditioned algorithm (van der Vorst)
-// that Eigen's BiCGSTAB implements, with the scalars kept on the device and
-// reductions in a fixed order.
+// that Eigen's BiCGSTAB implements, with reductions in a fixed order.
+//
+// A linear solve is one cooperative launch (k_bicgstab): an iteration's two
+// matrix-vector products, its vector updates and its dot products are a few
+// microseconds of work each, so as separate launches (17 per iteration, with
+// a read of the residual by the host) an iteration took 105 us whatever its
+// size.  Inside one kernel the five points of an iteration where every block
+// needs every other's result are barriers over the resident blocks.  64^2
+// Euler WENO3 (16,384 rows of 36): 19 us per iteration, about half of it the
+// barriers and sums; two Crank-Nicolson steps (20 Newton, 489 BiCGSTAB
+// iterations) 66.7 -> 12.5 ms.  The FP64 units set the rest: with the
+// iteration's scalars divided on the FP64 pipe by every warp it took 24 us,
+// with every thread summing and one warp per scheduler 34 us.
 #include <cmath>
+#include <algorithm>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include <cuda_runtime.h>
 
+#include "numerics.cuh"
 #include "problem_impl.hpp"
 
 namespace pda {
 namespace impl {
 
-constexpr int RB = 256;      // threads per reduction block
-constexpr int NRED = 1024;   // reduction blocks (grid-stride)
+constexpr int RB = 512;       // threads per block of the solver
+constexpr int LPR = 4;        // lanes per matrix row: 9 to 95 entries a row
+constexpr int MAX_BLOCKS = 2048;
 
-// ----------------------------------------------------------- vector kernels
-__global__ void k_residual(int scheme, long n, const double *__restrict__ y, const double *__restrict__ yn,
-                           const double *__restrict__ f, const double *__restrict__ fn, double dt,
-                           double *__restrict__ R) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (scheme == 0) R[i] = y[i] - yn[i] - dt * f[i];
-  else R[i] = y[i] - yn[i] - (dt / 2.) * (f[i] + fn[i]);
-}
-
-// J_R = I + c Jf in place of a copy of Jf's values; diag[i] = J_R(i, i)
-__global__ void k_jr_values(long rows, const int *__restrict__ rowptr, const int *__restrict__ colidx,
-                            const double *__restrict__ J, double c, double *__restrict__ JR,
-                            double *__restrict__ diag) {
-  const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  double d = 1.;
-  for (int q = rowptr[r]; q < rowptr[r + 1]; ++q) {
+// System of one Newton iteration: R, J_R = I + c Jf in place of Jf's values,
+// and the reciprocals of J_R's diagonal.  LPR lanes per row.
+__global__ void __launch_bounds__(256)
+k_system(int scheme, long n, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+         const double *__restrict__ y, const double *__restrict__ yn, const double *__restrict__ f,
+         const double *__restrict__ fn, double dt, double c, double *__restrict__ J, double *__restrict__ dinv,
+         double *__restrict__ R) {
+  const long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+  const int lane = threadIdx.x % LPR;
+  if (r >= n) return;
+  if (lane == 0) {
+    if (scheme == 0) R[r] = y[r] - yn[r] - dt * f[r];
+    else R[r] = y[r] - yn[r] - (dt / 2.) * (f[r] + fn[r]);
+  }
+  for (int q = rowptr[r] + lane; q < rowptr[r + 1]; q += LPR) {
     double v = c * J[q];
     if (colidx[q] == r) {
       v += 1.;
-      d = v;
+      dinv[r] = div_rn(1., v);
     }
-    JR[q] = v;
+    J[q] = v;
   }
-  diag[r] = d;
 }
 
-__global__ void k_spmv(long rows, const int *__restrict__ rowptr, const int *__restrict__ colidx,
-                       const double *__restrict__ A, const double *__restrict__ x, double *__restrict__ y) {
-  const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  double s = 0.;
-  for (int q = rowptr[r]; q < rowptr[r + 1]; ++q) s += A[q] * x[colidx[q]];
-  y[r] = s;
+__global__ void k_minus(long n, const double *__restrict__ x, double *__restrict__ y) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) y[i] -= x[i];
 }
 
-// block partial sums of a.b (fixed order inside each block)
-__global__ void __launch_bounds__(RB) k_dot_partial(long n, const double *__restrict__ a,
-                                                    const double *__restrict__ b, double *__restrict__ part) {
-  __shared__ double red[RB];
-  double s = 0.;
-  for (long i = (long)blockIdx.x * RB + threadIdx.x; i < n; i += (long)gridDim.x * RB) s += a[i] * b[i];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = RB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+// What the host reads after a solve.
+struct SolveInfo {
+  double rr, bb, dd;  // |r|^2, |b|^2, |x|^2
+  int iters;
+  int error;  // a barrier's wait ran out
+};
+
+struct SolveArgs {
+  long n;
+  const int *rowptr, *colidx;
+  const double *A, *dinv, *b;
+  double *x, *r, *p, *v, *s, *t, *y, *z;  // vectors written here
+  double *part;                           // [4][MAX_BLOCKS] block sums
+  unsigned *arrived;                      // barrier arrivals, zero at launch
+  SolveInfo *info;                        // zero at launch
+  double tol2;
+  int maxIt;
+};
+
+// Barrier over the resident blocks of a cooperative launch.  Arrivals count
+// up; each wait is bounded and a wait that runs out sets the error flag, on
+// which every block leaves.
+constexpr unsigned POLLS = 1u << 24;
+struct GridBarrier {
+  unsigned *arrived;
+  int *error;
+  unsigned target = 0;
+  __device__ bool sync() {
+    __shared__ int failed;
     __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-// out = sum of the partials (one block)
-__global__ void __launch_bounds__(RB) k_dot_final(int nparts, const double *__restrict__ part, double *out) {
-  __shared__ double red[RB];
-  double s = 0.;
-  for (int i = threadIdx.x; i < nparts; i += RB) s += part[i];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = RB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+      int bad = 0;
+      for (unsigned k = 0;; ++k) {
+        unsigned now;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(arrived) : "memory");
+        if ((int)(now - target) >= 0) break;
+        if (k >= POLLS || ((k & 1023u) == 1023u && *(volatile int *)error != 0)) {
+          atomicExch(error, 1);
+          bad = 1;
+          break;
+        }
+      }
+      failed = bad;
+    }
     __syncthreads();
+    return failed == 0;
   }
-  if (threadIdx.x == 0) *out = red[0];
+};
+
+// GB300 takes 64 cycles per FP64 warp instruction and scheduler, whatever its
+// active lanes, so sums are laid out for few of them: only warps that hold
+// values add, over no more lanes than hold them.
+// Sum over the lanes that are a multiple of STRIDE (the others hold zeros).
+template <int STRIDE>
+__device__ __forceinline__ double warp_sum(double s) {
+#pragma unroll
+  for (int o = 16; o >= STRIDE; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+// sums of v[0..N-1] over the block, to the block's places in part[0..N-1]; active: whether this warp holds any
+template <int STRIDE, int N>
+__device__ void block_sums(const double (&v)[N], bool active, double *part) {
+  constexpr int W = RB / 32;
+  __shared__ double red[N][W];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double w = active ? warp_sum<STRIDE>(v[k]) : 0.;
+    if (lane == 0) red[k][warp] = w;
+  }
+  __syncthreads();
+  if (warp < N) {
+    double w = lane < W ? red[warp][lane] : 0.;
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if (lane == 0) part[warp * MAX_BLOCKS + blockIdx.x] = w;
+  }
+}
+// the blocks' sums added up, the same in every block: warp k sum k
+template <int N>
+__device__ void grid_sums(const double *part, double (&v)[N]) {
+  __shared__ double tot[N];
+  static_assert(N <= RB / 32, "one warp per sum");
+  const int k = threadIdx.x / 32;
+  if (k < N) {
+    double w = 0.;
+    for (unsigned i = threadIdx.x % 32; i < gridDim.x; i += 32) w += __ldcg(part + k * MAX_BLOCKS + i);
+    w = warp_sum<1>(w);
+    if (threadIdx.x % 32 == 0) tot[k] = w;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = tot[i];
+  __syncthreads();
+}
+// row r of A times x, by LPR lanes (all lanes get the sum); a lane's loads go out in batches
+__device__ __forceinline__ double row_times(const SolveArgs &a, long r, int lane, const double *x) {
+  constexpr int UN = 9;
+  double s = 0.;
+  const int end = __ldg(a.rowptr + r + 1);
+  for (int q = __ldg(a.rowptr + r) + lane; q < end; q += UN * LPR) {
+    int c[UN];
+    double w[UN];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      const bool in = q + u * LPR < end;
+      c[u] = in ? __ldg(a.colidx + q + u * LPR) : -1;
+      w[u] = in ? __ldg(a.A + q + u * LPR) : 0.;
+    }
+    double g[UN];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) g[u] = c[u] >= 0 ? x[c[u]] : 0.;
+#pragma unroll
+    for (int u = 0; u < UN; ++u)
+      if (c[u] >= 0) s = fma(w[u], g[u], s);
+  }
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
+  return s;
 }
 
-// scalar slots of the solver state on the device
-enum Sc { RHO, RHO_OLD, ALPHA, OMEGA, BETA, R0V, TT, TS, RR, BB, NSC };
+// Solve A x = b from x = 0.  Cooperative launch, RB threads per block; a
+// block owns a run of consecutive rows.
+__global__ void __launch_bounds__(RB, 1) k_bicgstab(SolveArgs a) {
+  const long chunk = (a.n + gridDim.x - 1) / gridDim.x;
+  const long lo = chunk * blockIdx.x < a.n ? chunk * blockIdx.x : a.n, hi = lo + chunk < a.n ? lo + chunk : a.n;
+  const long own = lo + threadIdx.x;                      // vector entries own, own + RB, ... below hi
+  const bool active = lo + threadIdx.x / 32 * 32 < hi;    // this warp holds vector entries
+  const int lane = threadIdx.x % LPR;
+  const long warpRow = lo + threadIdx.x / 32 * (32 / LPR);  // first row of this warp's lane groups
+  const long group = lo + threadIdx.x / LPR;
+  const bool rowsHere = warpRow < hi;
+  GridBarrier bar{a.arrived, &a.info->error};
+  int phase = 0;
+  double *const parts[2] = {a.part, a.part + 2 * MAX_BLOCKS};  // one is read while the next is written
+  double one[1] = {0.}, two[2];
+  for (long i = own; i < hi; i += RB) {
+    const double bi = a.b[i];
+    a.r[i] = bi;
+    a.x[i] = 0.;
+    a.p[i] = 0.;
+    a.v[i] = 0.;
+    one[0] = fma(bi, bi, one[0]);
+  }
+  block_sums<1>(one, active, parts[phase]);
+  if (!bar.sync()) return;
+  grid_sums(parts[phase], one);
+  phase ^= 1;
+  const double bb = one[0];
+  double rr = bb, rho = 1., alpha = 1., omega = 1., rhoNext = bb, dd = 0.;
+  int it = 0;
+  if (bb > 0.) {
+    while (it < a.maxIt) {
+      ++it;
+      const double beta = div_rn(rhoNext, rho) * div_rn(alpha, omega);  // on the integer pipe
+      rho = rhoNext;
+      for (long i = own; i < hi; i += RB) {
+        const double pi = fma(beta, fma(-omega, a.v[i], a.p[i]), a.r[i]);
+        a.p[i] = pi;
+        a.y[i] = pi * a.dinv[i];
+      }
+      if (!bar.sync()) return;
+      one[0] = 0.;
+      for (long w = warpRow, r = group; w < hi; w += RB / LPR, r += RB / LPR) {
+        const double v = row_times(a, r < hi ? r : hi - 1, lane, a.y);
+        if (r < hi && lane == 0) {
+          a.v[r] = v;
+          one[0] = fma(a.b[r], v, one[0]);
+        }
+      }
+      block_sums<LPR>(one, rowsHere, parts[phase]);
+      if (!bar.sync()) return;
+      grid_sums(parts[phase], one);
+      phase ^= 1;
+      alpha = div_rn(rho, one[0]);
+      for (long i = own; i < hi; i += RB) {
+        const double si = fma(-alpha, a.v[i], a.r[i]);
+        a.s[i] = si;
+        a.z[i] = si * a.dinv[i];
+      }
+      if (!bar.sync()) return;
+      two[0] = two[1] = 0.;
+      for (long w = warpRow, r = group; w < hi; w += RB / LPR, r += RB / LPR) {
+        const double t = row_times(a, r < hi ? r : hi - 1, lane, a.z);
+        if (r < hi && lane == 0) {
+          a.t[r] = t;
+          two[0] = fma(t, t, two[0]);
+          two[1] = fma(t, a.s[r], two[1]);
+        }
+      }
+      block_sums<LPR>(two, rowsHere, parts[phase]);
+      if (!bar.sync()) return;
+      grid_sums(parts[phase], two);
+      phase ^= 1;
+      omega = two[0] > 0. ? div_rn(two[1], two[0]) : 0.;
+      two[0] = two[1] = 0.;
+      for (long i = own; i < hi; i += RB) {
+        a.x[i] += fma(alpha, a.y[i], omega * a.z[i]);
+        const double ri = fma(-omega, a.t[i], a.s[i]);
+        a.r[i] = ri;
+        two[0] = fma(ri, ri, two[0]);
+        two[1] = fma(a.b[i], ri, two[1]);
+      }
+      block_sums<1>(two, active, parts[phase]);
+      if (!bar.sync()) return;
+      grid_sums(parts[phase], two);
+      phase ^= 1;
+      rr = two[0];
+      rhoNext = two[1];
+      if (!(rr >= 0.) || rr <= a.tol2 * bb) break;
+    }
+    // |x|^2 (each thread sums the entries that it wrote)
+    one[0] = 0.;
+    for (long i = own; i < hi; i += RB) one[0] = fma(a.x[i], a.x[i], one[0]);
+    block_sums<1>(one, active, parts[phase]);
+    if (!bar.sync()) return;
+    grid_sums(parts[phase], one);
+    dd = one[0];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.info->rr = rr;
+    a.info->bb = bb;
+    a.info->dd = dd;
+    a.info->iters = it;
+  }
+}
 
-__global__ void k_beta(double *sc) {
-  // beta = (rho / rho_old) * (alpha / omega)
-  sc[BETA] = (sc[RHO] / sc[RHO_OLD]) * (sc[ALPHA] / sc[OMEGA]);
-}
-__global__ void k_alpha(double *sc) { sc[ALPHA] = sc[RHO] / sc[R0V]; }
-__global__ void k_omega(double *sc) { sc[OMEGA] = sc[TT] > 0. ? sc[TS] / sc[TT] : 0.; }
-__global__ void k_shift_rho(double *sc) { sc[RHO_OLD] = sc[RHO]; }
-
-// p = r + beta (p - omega v);  y = p / diag
-__global__ void k_update_p(long n, const double *__restrict__ r, const double *__restrict__ v,
-                           const double *__restrict__ diag, const double *__restrict__ sc, double *__restrict__ p,
-                           double *__restrict__ y) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double pi = r[i] + sc[BETA] * (p[i] - sc[OMEGA] * v[i]);
-  p[i] = pi;
-  y[i] = pi / diag[i];
-}
-
-// s = r - alpha v;  z = s / diag
-__global__ void k_update_s(long n, const double *__restrict__ r, const double *__restrict__ v,
-                           const double *__restrict__ diag, const double *__restrict__ sc, double *__restrict__ s,
-                           double *__restrict__ z) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double si = r[i] - sc[ALPHA] * v[i];
-  s[i] = si;
-  z[i] = si / diag[i];
-}
-
-// x += alpha y + omega z;  r = s - omega t
-__global__ void k_update_xr(long n, const double *__restrict__ y, const double *__restrict__ z,
-                            const double *__restrict__ s, const double *__restrict__ t,
-                            const double *__restrict__ sc, double *__restrict__ x, double *__restrict__ r) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  x[i] += sc[ALPHA] * y[i] + sc[OMEGA] * z[i];
-  r[i] = s[i] - sc[OMEGA] * t[i];
-}
-
-__global__ void k_copy(long n, const double *__restrict__ a, double *__restrict__ b) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = a[i];
-}
-__global__ void k_fill(long n, double v, double *__restrict__ b) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = v;
-}
-__global__ void k_axpy(long n, double a, const double *__restrict__ x, double *__restrict__ y) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] += a * x[i];
-}
-
+// Device buffers of the solver, kept by the problem that uses them.
 struct Work {
-  DevBuf<double> Un, Vn, V, J, JR, diag, R, d, r, r0, p, v, s, t, y, z, part, sc;
+  DevBuf<double> Un, Vn, V, J, dinv, R, d, r, p, v, s, t, y, z, part;
+  DevBuf<unsigned> arrived;
+  DevBuf<SolveInfo> info;
+  int blocks = 0;
+  void prepare(long n, long nnz) {
+    for (auto *b : {&Un, &Vn, &V, &dinv, &R, &d, &r, &p, &v, &s, &t, &y, &z}) b->alloc((size_t)n);
+    J.alloc((size_t)nnz);
+    part.alloc(4 * MAX_BLOCKS);
+    arrived.alloc(1);
+    info.alloc(1);
+    // every block resident: as many as the SMs hold, no more than the rows fill
+    int dev = 0, sms = 0, occ = 0;
+    PDA_CUDA(cudaGetDevice(&dev));
+    PDA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    PDA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bicgstab, RB, 0));
+    // barriers and sums cost with the blocks, latency without them: one block per SM up to four rounds of
+    // rows, then as many as stay resident
+    const long want = (n * LPR + RB - 1) / RB;
+    const long perSm = want <= 4l * sms ? 1 : std::max(occ, 1);
+    blocks = (int)std::max<long>(std::min({want, perSm * sms, (long)MAX_BLOCKS}), 1);
+  }
 };
 
 unsigned g1(long n) { return (unsigned)((n + 255) / 256); }
 
-void dot(Work &w, long n, const double *a, const double *b, int slot, cudaStream_t st) {
-  k_dot_partial<<<NRED, RB, 0, st>>>(n, a, b, w.part.p);
-  k_dot_final<<<1, RB, 0, st>>>(NRED, w.part.p, w.sc.p + slot);
-}
-
-double read_scalar(Work &w, int slot, cudaStream_t st) {
-  double h = 0.;
-  PDA_CUDA(cudaMemcpyAsync(&h, w.sc.p + slot, sizeof(double), cudaMemcpyDeviceToHost, st));
-  PDA_CUDA(cudaStreamSynchronize(st));
-  return h;
-}
-
-// solve JR d = R (x0 = 0); returns iterations, relres in *relres
+// solve J_R d = R (x0 = 0); *dd = |d|^2, *relres the relative residual
 int bicgstab(Work &w, long n, const int *rowptr, const int *colidx, double tol, int maxIt, cudaStream_t st,
-             double *relres) {
-  double *x = w.d.p;
-  k_fill<<<g1(n), 256, 0, st>>>(n, 0., x);
-  k_copy<<<g1(n), 256, 0, st>>>(n, w.R.p, w.r.p);
-  k_copy<<<g1(n), 256, 0, st>>>(n, w.R.p, w.r0.p);
-  k_fill<<<g1(n), 256, 0, st>>>(n, 0., w.p.p);
-  k_fill<<<g1(n), 256, 0, st>>>(n, 0., w.v.p);
-  const double one = 1.;
-  for (int s : {RHO, ALPHA, OMEGA})
-    PDA_CUDA(cudaMemcpyAsync(w.sc.p + s, &one, sizeof(double), cudaMemcpyHostToDevice, st));
-  dot(w, n, w.R.p, w.R.p, BB, st);
-  const double bb = read_scalar(w, BB, st);
-  if (!(bb > 0.)) {
-    *relres = 0.;
-    return 0;
-  }
-  int it = 0;
-  double rr = bb;
-  while (it < maxIt) {
-    ++it;
-    k_shift_rho<<<1, 1, 0, st>>>(w.sc.p);
-    dot(w, n, w.r0.p, w.r.p, RHO, st);
-    k_beta<<<1, 1, 0, st>>>(w.sc.p);
-    k_update_p<<<g1(n), 256, 0, st>>>(n, w.r.p, w.v.p, w.diag.p, w.sc.p, w.p.p, w.y.p);
-    k_spmv<<<g1(n), 256, 0, st>>>(n, rowptr, colidx, w.JR.p, w.y.p, w.v.p);
-    dot(w, n, w.r0.p, w.v.p, R0V, st);
-    k_alpha<<<1, 1, 0, st>>>(w.sc.p);
-    k_update_s<<<g1(n), 256, 0, st>>>(n, w.r.p, w.v.p, w.diag.p, w.sc.p, w.s.p, w.z.p);
-    k_spmv<<<g1(n), 256, 0, st>>>(n, rowptr, colidx, w.JR.p, w.z.p, w.t.p);
-    dot(w, n, w.t.p, w.t.p, TT, st);
-    dot(w, n, w.t.p, w.s.p, TS, st);
-    k_omega<<<1, 1, 0, st>>>(w.sc.p);
-    k_update_xr<<<g1(n), 256, 0, st>>>(n, w.y.p, w.z.p, w.s.p, w.t.p, w.sc.p, x, w.r.p);
-    dot(w, n, w.r.p, w.r.p, RR, st);
-    rr = read_scalar(w, RR, st);
-    if (!(rr >= 0.) || rr <= tol * tol * bb) break;
-  }
-  PDA_CUDA(cudaGetLastError());
-  *relres = std::sqrt(rr / bb);
-  return it;
+             double *relres, double *dd) {
+  PDA_CUDA(cudaMemsetAsync(w.arrived.p, 0, sizeof(unsigned), st));
+  PDA_CUDA(cudaMemsetAsync(w.info.p, 0, sizeof(SolveInfo), st));
+  SolveArgs a{n,      rowptr, colidx, w.J.p, w.dinv.p, w.R.p,     w.d.p,       w.r.p,    w.p.p,     w.v.p,
+              w.s.p,  w.t.p,  w.y.p,  w.z.p, w.part.p, w.arrived.p, w.info.p, tol * tol, maxIt};
+  void *args[] = {&a};
+  PDA_CUDA(cudaLaunchCooperativeKernel((const void *)k_bicgstab, dim3((unsigned)w.blocks), dim3(RB), args, 0, st));
+  SolveInfo h{};
+  PDA_CUDA(cudaMemcpyAsync(&h, w.info.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  PDA_CUDA(cudaStreamSynchronize(st));
+  if (h.error) throw Error(PDA_ERR_INTERNAL, "BiCGSTAB: a wait between thread blocks ran out");
+  *dd = h.dd;
+  *relres = h.bb > 0. ? std::sqrt(h.rr / h.bb) : 0.;
+  return h.iters;
 }
 
 }  // namespace impl
@@ -233,13 +367,9 @@ pda_status pda_advance_implicit(pda_problem *p, double *d_U, double t0, double d
   int64_t rows = 0, cols = 0, nnz = 0;
   pda_status st = pda_jacobian_shape(p, &rows, &cols, &nnz);
   if (st != PDA_OK) throw Error(st, pda_last_error());
-  pda::impl::Work w;
-  for (auto *b : {&w.Un, &w.Vn, &w.V, &w.diag, &w.R, &w.d, &w.r, &w.r0, &w.p, &w.v, &w.s, &w.t, &w.y, &w.z})
-    b->alloc((size_t)n);
-  w.J.alloc((size_t)nnz);
-  w.JR.alloc((size_t)nnz);
-  w.part.alloc(pda::impl::NRED);
-  w.sc.alloc(pda::impl::NSC);
+  if (!P.implicitWork) P.implicitWork = std::make_shared<pda::impl::Work>();
+  pda::impl::Work &w = *std::static_pointer_cast<pda::impl::Work>(P.implicitWork);
+  w.prepare(n, (long)nnz);
   cudaStream_t s = P.stream;
   pda::ensure_device_pattern(P);
   const int *rowptr = P.d_rowptr.p, *colidx = P.d_colidx.p;
@@ -247,7 +377,7 @@ pda_status pda_advance_implicit(pda_problem *p, double *d_U, double t0, double d
   double worstRel = 0.;
   double t = t0;
   for (int64_t step = 0; step < n_steps; ++step) {
-    pda::impl::k_copy<<<pda::impl::g1(n), 256, 0, s>>>(n, d_U, w.Un.p);
+    PDA_CUDA(cudaMemcpyAsync(w.Un.p, d_U, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     if (scheme == 1) {
       st = pda_velocity(p, w.Un.p, t, w.Vn.p);
       if (st != PDA_OK) throw Error(st, pda_last_error());
@@ -257,15 +387,14 @@ pda_status pda_advance_implicit(pda_problem *p, double *d_U, double t0, double d
     for (; it < newton_max_iters; ++it) {
       st = pda_velocity_and_jacobian(p, d_U, t + dt, w.V.p, w.J.p);
       if (st != PDA_OK) throw Error(st, pda_last_error());
-      pda::impl::k_residual<<<pda::impl::g1(n), 256, 0, s>>>(scheme, n, d_U, w.Un.p, w.V.p, w.Vn.p, dt, w.R.p);
-      pda::impl::k_jr_values<<<pda::impl::g1(n), 256, 0, s>>>(n, rowptr, colidx, w.J.p, c, w.JR.p, w.diag.p);
-      double rel = 0.;
-      totalLinear += pda::impl::bicgstab(w, n, rowptr, colidx, linear_tol, linear_max_iters, s, &rel);
+      pda::impl::k_system<<<pda::impl::g1(n * pda::impl::LPR), 256, 0, s>>>(
+          scheme, n, rowptr, colidx, d_U, w.Un.p, w.V.p, w.Vn.p, dt, c, w.J.p, w.dinv.p, w.R.p);
+      PDA_CUDA(cudaGetLastError());
+      double rel = 0., dd = 0.;
+      totalLinear += pda::impl::bicgstab(w, n, rowptr, colidx, linear_tol, linear_max_iters, s, &rel, &dd);
       worstRel = std::max(worstRel, rel);
-      pda::impl::dot(w, n, w.d.p, w.d.p, pda::impl::RR, s);
-      const double dd = pda::impl::read_scalar(w, pda::impl::RR, s);
       if (std::sqrt(dd) < newton_tol) break;  // stop before updating, as Pressio does
-      pda::impl::k_axpy<<<pda::impl::g1(n), 256, 0, s>>>(n, -1., w.d.p, d_U);
+      pda::impl::k_minus<<<pda::impl::g1(n), 256, 0, s>>>(n, w.d.p, d_U);
     }
     totalNewton += it + 1;
     maxNewton = std::max(maxNewton, it + 1);

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <new>
 #include <string>
+#include <memory>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -192,6 +193,7 @@ struct pda_problem {
   // host-buffer entry points and steppers
   pda::DevBuf<double> d_U, d_V, d_J;
   pda::DevBuf<double> aux, r[4];
+  std::shared_ptr<void> implicitWork;  // implicit stepper's device buffers (implicit.cu), from its first call
   cudaGraphExec_t stepGraph = nullptr;
   int stepGraphKind = -1;
   double stepGraphDt = 0;
