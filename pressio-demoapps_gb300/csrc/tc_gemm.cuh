@@ -294,6 +294,8 @@ __device__ __forceinline__ void tile_epilogue(uint32_t tmem, int KT, long M, lon
     }
   } else if (KT > 0) {
     const long row = m0 + warp * 32 + lane;
+    auto aligned = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    const bool vec = N % 8 == 0 && aligned(partial) && aligned(outF) && aligned(outB) && aligned(preact) && aligned(bias);
 #pragma unroll 1
     for (int c0 = 0; c0 < BN_ && n0 + c0 < N; c0 += 16) {  // column groups that hold output columns
       uint32_t r[16];
@@ -305,17 +307,63 @@ __device__ __forceinline__ void tile_epilogue(uint32_t tmem, int KT, long M, lon
             "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
           : "r"(taddr));
       asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      // a thread's 16 columns are consecutive: whole 16-byte pieces of the output rows where N and the
+      // bases allow them (one column at a time, the stores of 32 rows took 50 us of a 52 us launch at
+      // 128 x 256 x 64)
+      const long cb = n0 + c0;
+      const bool whole = vec && cb + 16 <= N;
       if (row < M && partial) {
-        float *pp = partial + row * N;
+        float *pp = partial + row * N + cb;
+        if (whole) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const long col = n0 + c0 + j;
-          if (col < N) pp[col] = __uint_as_float(r[j]);
+          for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4 *>(pp + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
+                                                              __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (cb + j < N) pp[j] = __uint_as_float(r[j]);
+        }
+      } else if (row < M && whole) {
+        float v[16];
+        const long base = row * N + cb;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+        if (epi != EPI_NONE) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) {
+            const float4 b4 = __ldg(reinterpret_cast<const float4 *>(bias + cb + j));
+            v[j] += b4.x;
+            v[j + 1] += b4.y;
+            v[j + 2] += b4.z;
+            v[j + 3] += b4.w;
+          }
+        }
+        if (preact) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4 *>(preact + base + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+        if (epi == EPI_BIAS_ELU) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = elu(v[j]);
+        }
+        if (outF) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4 *>(outF + base + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+        if (outB) {
+          __align__(16) __nv_bfloat16 hb[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) hb[j] = __float2bfloat16_rn(v[j]);
+          reinterpret_cast<uint4 *>(outB + base)[0] = reinterpret_cast<const uint4 *>(hb)[0];
+          reinterpret_cast<uint4 *>(outB + base)[1] = reinterpret_cast<const uint4 *>(hb)[1];
         }
       } else if (row < M) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const long col = n0 + c0 + j;
+          const long col = cb + j;
           if (col < N) {
             float v = __uint_as_float(r[j]);
             if (epi != EPI_NONE) v += bias[col];
