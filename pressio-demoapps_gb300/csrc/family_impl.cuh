@@ -24,21 +24,21 @@ constexpr bool F_dim_ok(int axis) { return axis < Fam<PDA_FAM>::dim; }
 
 template <int SCHEME>
 void rows_velocity_s(const RowTable &ta, const RowTable &tb, const MeshArgs &m, const Phys &p, const double *U,
-                     double *V, cudaStream_t s) {
+                     double *V, const StageArgs &st, cudaStream_t s) {
   const int rows = ta.nrows + tb.nrows;
   if (rows <= 0) return;
   // rows per block: the fewest blocks that still cover every SM once
   const int rpb = std::max(1, std::min(VelPar<FAM>::RPB_MAX, div_up(rows, device_sms())));
   const int nbA = div_up(ta.nrows, rpb), nb = nbA + div_up(tb.nrows, rpb);
-  k_rows_velocity_par<FAM, SCHEME><<<nb, VelPar<FAM>::THREADS, 0, s>>>(ta, tb, nbA, rpb, m, p, U, V);
+  k_rows_velocity_par<FAM, SCHEME><<<nb, VelPar<FAM>::THREADS, 0, s>>>(ta, tb, nbA, rpb, m, p, U, V, st);
 }
 
 void rows_velocity(int scheme, const RowTable &ta, const RowTable &tb, const MeshArgs &m, const Phys &p,
-                   const double *U, double *V, cudaStream_t s) {
+                   const double *U, double *V, const StageArgs &st, cudaStream_t s) {
   switch (scheme) {
-    case FirstOrder: rows_velocity_s<FirstOrder>(ta, tb, m, p, U, V, s); break;
-    case Weno3: rows_velocity_s<Weno3>(ta, tb, m, p, U, V, s); break;
-    default: rows_velocity_s<Weno5>(ta, tb, m, p, U, V, s); break;
+    case FirstOrder: rows_velocity_s<FirstOrder>(ta, tb, m, p, U, V, st, s); break;
+    case Weno3: rows_velocity_s<Weno3>(ta, tb, m, p, U, V, st, s); break;
+    default: rows_velocity_s<Weno5>(ta, tb, m, p, U, V, st, s); break;
   }
 }
 
@@ -78,7 +78,7 @@ void struct_velocity_s(const Box &b, const MeshArgs &m, const Phys &p, const dou
     faces_s<SCHEME, 0>(b, p, U, Fb[0], s, launches, ev);
     if constexpr (F::dim > 1) faces_s<SCHEME, 1>(b, p, U, Fb[1], s, launches, ev);
     if constexpr (F::dim > 2) faces_s<SCHEME, 2>(b, p, U, Fb[2], s, launches, ev);
-    k_struct_balance<FAM><<<div_up(nc, 256), 256, 0, s>>>(b, m, p, U, Fb[0], Fb[1], Fb[2], V);
+    k_struct_balance<FAM><<<div_up(nc, 256), 256, 0, s>>>(b, m, p, U, Fb[0], Fb[1], Fb[2], V, StageArgs{});
     ++*launches;
   }
   if (ev) cudaEventRecord(ev[F::dim + 1], s);
@@ -109,10 +109,10 @@ void struct_faces(int scheme, int axis, const Box &b, const Phys &p, const doubl
 }
 
 void struct_balance(const Box &b, const MeshArgs &m, const Phys &p, const double *U, const double *const F[3],
-                    double *V, cudaStream_t s) {
+                    double *V, const StageArgs &st, cudaStream_t s) {
   long nc = 1;
   for (int a = 0; a < 3; ++a) nc *= (long)(b.hi[a] - b.lo[a]);
-  if (nc > 0) k_struct_balance<FAM><<<div_up(nc, 256), 256, 0, s>>>(b, m, p, U, F[0], F[1], F[2], V);
+  if (nc > 0) k_struct_balance<FAM><<<div_up(nc, 256), 256, 0, s>>>(b, m, p, U, F[0], F[1], F[2], V, st);
 }
 
 void rows_vj_inner(int scheme, const RowTable &t, const MeshArgs &m, const Phys &p, const double *U,

@@ -448,25 +448,31 @@ __device__ __forceinline__ bool balance_values(const Box &b, const MeshArgs &m, 
   return true;
 }
 
+__device__ __forceinline__ void put_velocity(double *V, size_t q, double v, const StageArgs &st) {
+  if (st.kind < 0) V[q] = v;
+  else if (st.kind == 0) st.out[q] = st.x[q] + st.cb * v;
+  else st.out[q] = st.ca * st.y[q] + st.cb * st.x[q] + st.cc * v;
+}
+
 template <int FAM>
 __device__ __forceinline__ void balance_cell(const Box &b, const MeshArgs &m, const Phys &p,
                                              const double *__restrict__ U, const double *__restrict__ Fx,
                                              const double *__restrict__ Fy, const double *__restrict__ Fz,
-                                             double *__restrict__ V, long t) {
+                                             double *V, long t, const StageArgs &st = StageArgs{}) {
   constexpr int NDPC = Fam<FAM>::ndpc;
   double v[NDPC];
   long cell;
   if (!balance_values<FAM>(b, m, p, U, Fx, Fy, Fz, t, v, cell)) return;
 #pragma unroll
-  for (int d = 0; d < NDPC; ++d) V[cell * NDPC + d] = v[d];
+  for (int d = 0; d < NDPC; ++d) put_velocity(V, cell * NDPC + d, v[d], st);
 }
 
 template <int FAM>
 __global__ void __launch_bounds__(256)
 k_struct_balance(Box b, MeshArgs m, Phys p, const double *__restrict__ U,
                  const double *__restrict__ Fx, const double *__restrict__ Fy,
-                 const double *__restrict__ Fz, double *__restrict__ V) {
-  balance_cell<FAM>(b, m, p, U, Fx, Fy, Fz, V, (long)blockIdx.x * blockDim.x + threadIdx.x);
+                 const double *__restrict__ Fz, double *V, StageArgs st) {
+  balance_cell<FAM>(b, m, p, U, Fx, Fy, Fz, V, (long)blockIdx.x * blockDim.x + threadIdx.x, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -852,7 +858,7 @@ template <int FAM> struct VelFace {
 template <int FAM, int SCHEME>
 __global__ void __launch_bounds__(VelPar<FAM>::THREADS)
 k_rows_velocity_par(RowTable ta, RowTable tb, int nbA, int rpb, MeshArgs m, Phys p, const double *__restrict__ U,
-                    double *__restrict__ V) {
+                    double *V, StageArgs st) {
   using F = Fam<FAM>;
   using VP = VelPar<FAM>;
   constexpr int NDPC = F::ndpc, DIM = F::dim, H = SchemeTraits<SCHEME>::h, S = 2 * H + 1, G = 2 * H;
@@ -918,7 +924,7 @@ k_rows_velocity_par(RowTable ta, RowTable tb, int nbA, int rpb, MeshArgs m, Phys
         if (k == 1) vk -= div_rn(p.coriolis * u2, u0);
         if (k == 2) vk += div_rn(p.coriolis * u1, u0);
       }
-      V[(size_t)t.rows[e] * NDPC + k] = vk;
+      put_velocity(V, (size_t)t.rows[e] * NDPC + k, vk, st);
     }
   }
 }

@@ -8,9 +8,10 @@
 namespace pda {
 
 struct Launchers {
-  // velocity of the rows of one or two row tables (tb may be empty), one launch
+  // velocity of the rows of one or two row tables (tb may be empty), one launch;
+  // st: what becomes of it
   void (*rows_velocity)(int scheme, const RowTable &ta, const RowTable &tb, const MeshArgs &m, const Phys &p,
-                        const double *U, double *V, cudaStream_t s);
+                        const double *U, double *V, const StageArgs &st, cudaStream_t s);
   // structured interior: faces once per axis into F[axis], then balance into V
   // ev (may be null): dim+2 events recorded before the first face launch,
   // after each face launch and after the balance launch
@@ -23,7 +24,7 @@ struct Launchers {
   void (*struct_faces)(int scheme, int axis, const Box &b, const Phys &p, const double *U, double *F,
                        cudaStream_t s);
   void (*struct_balance)(const Box &b, const MeshArgs &m, const Phys &p, const double *U,
-                         const double *const F[3], double *V, cudaStream_t s);
+                         const double *const F[3], double *V, const StageArgs &st, cudaStream_t s);
   // V and J for inner rows / near-boundary rows
   void (*rows_vj_inner)(int scheme, const RowTable &t, const MeshArgs &m, const Phys &p,
                         const double *U, const int *rowptr, double *V, double *J, cudaStream_t s);

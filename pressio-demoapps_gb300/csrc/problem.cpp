@@ -706,7 +706,9 @@ void join_side(pda_problem &P) {
 }
 
 // --------------------------------------------------------------- evaluation
-void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t *ev = nullptr) {
+// V at (U, t), or with st the explicit stage that consumes it (V unused)
+void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t *ev = nullptr,
+              const StageArgs &st = StageArgs{}) {
   check_evaluable(P);
   sync_recipes(P);
   MeshArgs ma = P.margs;
@@ -721,20 +723,19 @@ void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t 
       Fb[a] = P.F[a].p;
     }
     int nl = 0;
-    if (!ev && P.dim >= 2) {
+    if (!ev && (P.dim >= 2 || st.kind >= 0)) {
       // the face passes of different axes are independent (separate face
       // arrays): the y faces run on the side stream beside the x (and z)
       // faces, so each pass's last, partly filled wave overlaps the other's
-      // (1024^2 Riemann WENO5: 1.302 ms per velocity against 1.319 ms with
-      // the passes in sequence).  The profiling path (ev) keeps the
-      // sequence, one pass at a time.
-      fork_side(P);
+      // (measured on 1024^2 Riemann WENO5 with earlier face kernels: 1.302 ms
+      // per velocity against 1.319 ms in sequence).  The profiling path (ev)
+      // keeps the sequence, one pass at a time.
+      if (P.dim >= 2) P.L->struct_faces(P.scheme, 1, b, P.phys, U, Fb[1], fork_side(P));
       P.L->struct_faces(P.scheme, 0, b, P.phys, U, Fb[0], P.stream);
-      P.L->struct_faces(P.scheme, 1, b, P.phys, U, Fb[1], P.side);
       if (P.dim == 3) P.L->struct_faces(P.scheme, 2, b, P.phys, U, Fb[2], P.stream);
-      join_side(P);
+      if (P.dim >= 2) join_side(P);
       const double *Fc[3] = {Fb[0], Fb[1], Fb[2]};
-      P.L->struct_balance(b, ma, P.phys, U, Fc, V, P.stream);
+      P.L->struct_balance(b, ma, P.phys, U, Fc, V, st, P.stream);
       check_launch(P, P.dim + 1);
     } else {
       P.L->struct_velocity(P.scheme, b, ma, P.phys, U, Fb, V, P.stream, &nl, ev);
@@ -752,7 +753,7 @@ void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t 
   const RowTable &ta = P.useStruct ? none : P.innerT.t;
   const RowTable &tb = P.structAll ? none : P.nearT.t;
   if (ta.nrows + tb.nrows > 0) {
-    P.L->rows_velocity(P.scheme, ta, tb, ma, P.phys, U, V, P.stream);
+    P.L->rows_velocity(P.scheme, ta, tb, ma, P.phys, U, V, st, P.stream);
     check_launch(P);
   }
   if (ev) cudaEventRecord(ev[P.dim + 2], P.stream);
@@ -1062,29 +1063,25 @@ void create_problem(pda_problem &P, const Mesh &m, int family, int probEn, int s
 // ------------------------------------------------------------------ steppers
 namespace {
 
+constexpr int kGraphSteps = 16;  // steps per launch of the graph of several steps
+
 void stepper_buffers(pda_problem &P, int nr) {
   P.aux.alloc(P.dofsStencil);
   for (int i = 0; i < nr; ++i) P.r[i].alloc(P.dofsSample);
 }
 
 // One step of SSP-RK3 (ode_explicit_stepper_without_mass_matrix.hpp:230-282).
+// Each stage is part of the evaluation that it consumes (StageArgs); the
+// second writes beside its state, whose other cells are still read.  1000
+// cells: 14.5 -> 9.6 us per step, whose six launches were as long as their work.
 void ssprk3_step(pda_problem &P, double *U, double t, double dt) {
-  const long n = (long)P.dofsStencil;
-  double *r0 = P.r[0].p, *aux = P.aux.p;
+  double *a = P.aux.p, *b = P.r[0].p;
   const double tHalf = t + dt / 2., tNext = t + dt;
-  velocity(P, U, r0, t);
-  launch_axpby_stage(0, aux, U, r0, nullptr, 0., dt, 0., 0., nullptr, nullptr, n, P.stream);
-  check_launch(P);
-  velocity(P, aux, r0, tNext);
+  velocity(P, U, nullptr, t, nullptr, StageArgs{0, a, U, nullptr, 0., dt, 0.});
   const double fourInv = 1. / 4., threeOvFour = 3. / 4.;
-  launch_axpby_stage(1, aux, U, r0, nullptr, fourInv, threeOvFour, fourInv * dt, 0., nullptr, nullptr, n,
-                     P.stream);
-  check_launch(P);
-  velocity(P, aux, r0, tHalf);
+  velocity(P, a, nullptr, tNext, nullptr, StageArgs{1, b, U, a, fourInv, threeOvFour, fourInv * dt});
   const double oneOvThree = 1. / 3., twoOvThree = 2. / 3.;
-  launch_axpby_stage(1, U, aux, r0, nullptr, oneOvThree, twoOvThree, twoOvThree * dt, 0., nullptr, nullptr,
-                     n, P.stream);
-  check_launch(P);
+  velocity(P, b, nullptr, tHalf, nullptr, StageArgs{1, U, b, U, oneOvThree, twoOvThree, twoOvThree * dt});
 }
 
 // One step of RK4 (ode_explicit_stepper_without_mass_matrix.hpp:284-336).
@@ -1126,35 +1123,49 @@ void advance(pda_problem &P, int kind, double *U, double t0, double dt, int64_t 
     }
     return;
   }
-  // Capture one step and replay it: the kernels do not depend on t for these
-  // boundary conditions.  The graph bakes in U and dt.
-  if (P.stepGraph && (P.stepGraphKind != kind || P.stepGraphDt != dt || P.stepGraphU != U)) {
-    cudaGraphExecDestroy(P.stepGraph);
-    P.stepGraph = nullptr;
+  // Capture steps and replay them: the kernels do not depend on t for these
+  // boundary conditions.  The graphs bake in U and dt.  Launching a graph
+  // costs the host about 13 us, as long as a step of a small problem, so runs
+  // of at least 2 kGraphSteps steps go out kGraphSteps at a time (1D, 1000
+  // cells: 13.3 us per step one at a time).
+  if (P.stepGraphKind != kind || P.stepGraphDt != dt || P.stepGraphU != U) {
+    for (cudaGraphExec_t *g : {&P.stepGraph, &P.stepsGraph}) {
+      if (*g) cudaGraphExecDestroy(*g);
+      *g = nullptr;
+    }
+    P.stepGraphKind = kind;
+    P.stepGraphDt = dt;
+    P.stepGraphU = U;
   }
-  if (!P.stepGraph) {
-    // lazily built tables and buffers must exist before capture
-    velocity(P, U, P.r[0].p, t0);
-    PDA_CUDA(cudaStreamSynchronize(P.stream));
+  auto capture = [&](int steps) {
     cudaGraph_t g;
+    cudaGraphExec_t exec = nullptr;
     PDA_CUDA(cudaStreamBeginCapture(P.stream, cudaStreamCaptureModeThreadLocal));
     const int64_t before = P.launches;
     try {
-      step(t0);
+      for (int k = 0; k < steps; ++k) step(t0);
     } catch (...) {
       cudaStreamEndCapture(P.stream, &g);
       throw;
     }
     PDA_CUDA(cudaStreamEndCapture(P.stream, &g));
-    P.stepGraphLaunches = P.launches - before;
+    P.stepGraphLaunches = (P.launches - before) / steps;
     P.launches = before;
-    PDA_CUDA(cudaGraphInstantiate(&P.stepGraph, g, 0));
+    const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
-    P.stepGraphKind = kind;
-    P.stepGraphDt = dt;
-    P.stepGraphU = U;
+    PDA_CUDA(e);
+    return exec;
+  };
+  const int64_t many = nsteps >= 2 * kGraphSteps ? nsteps / kGraphSteps : 0, single = nsteps - many * kGraphSteps;
+  if ((many && !P.stepsGraph) || (single && !P.stepGraph)) {
+    // lazily built tables and buffers must exist before capture
+    velocity(P, U, P.r[0].p, t0);
+    PDA_CUDA(cudaStreamSynchronize(P.stream));
+    if (many && !P.stepsGraph) P.stepsGraph = capture(kGraphSteps);
+    if (single && !P.stepGraph) P.stepGraph = capture(1);
   }
-  for (int64_t s = 0; s < nsteps; ++s) PDA_CUDA(cudaGraphLaunch(P.stepGraph, P.stream));
+  for (int64_t s = 0; s < many; ++s) PDA_CUDA(cudaGraphLaunch(P.stepsGraph, P.stream));
+  for (int64_t s = 0; s < single; ++s) PDA_CUDA(cudaGraphLaunch(P.stepGraph, P.stream));
   P.launches += nsteps * P.stepGraphLaunches;
 }
 
@@ -1375,7 +1386,7 @@ pda_status pda_velocity_noalloc(pda_problem *p, const double *dU, double t, doub
                 PDA_ERR_UNSUPPORTED,
                 "pda_velocity_noalloc: full meshes only, and the row tables of this problem are not on the device "
                 "yet; one pda_velocity call on the problem uploads them");
-    P.L->rows_velocity(P.scheme, P.innerT.t, P.nearT.t, ma, P.phys, dU, dV, P.stream);
+    P.L->rows_velocity(P.scheme, P.innerT.t, P.nearT.t, ma, P.phys, dU, dV, pda::StageArgs{}, P.stream);
     pda::check_launch(P);
     return PDA_OK;
   }
@@ -1409,7 +1420,7 @@ pda_status pda_velocity_noalloc(pda_problem *p, const double *dU, double t, doub
   pda::check_launch(P, nl);
   if (!P.structAll && P.nearT.t.nrows > 0) {
     pda::RowTable none{};
-    P.L->rows_velocity(P.scheme, none, P.nearT.t, ma, P.phys, dU, dV, P.stream);
+    P.L->rows_velocity(P.scheme, none, P.nearT.t, ma, P.phys, dU, dV, pda::StageArgs{}, P.stream);
     pda::check_launch(P);
   }
   PDA_API_END
@@ -1542,7 +1553,7 @@ bool velocity_host_banded(pda_problem &P, const double *hU, double t, double *hV
     bb.lo[1] = r[b];
     bb.hi[1] = r[b + 1];
     const double *Fb[3] = {Fx + (size_t)(nx + 1) * r[b] * nd, Fy + (size_t)nx * r[b] * nd, nullptr};
-    P.L->struct_balance(bb, ma, P.phys, U, Fb, V, cs[b]);
+    P.L->struct_balance(bb, ma, P.phys, U, Fb, V, StageArgs{}, cs[b]);
     PDA_CUDA(cudaEventRecord(evBal[b], cs[b]));
   }
   for (int b = 0; b < NB; ++b) {

@@ -194,7 +194,7 @@ struct pda_problem {
   pda::DevBuf<double> d_U, d_V, d_J;
   pda::DevBuf<double> aux, r[4];
   std::shared_ptr<void> implicitWork;  // implicit stepper's device buffers (implicit.cu), from its first call
-  cudaGraphExec_t stepGraph = nullptr;
+  cudaGraphExec_t stepGraph = nullptr, stepsGraph = nullptr;  // one step, several steps
   int stepGraphKind = -1;
   double stepGraphDt = 0;
   double *stepGraphU = nullptr;
@@ -202,6 +202,7 @@ struct pda_problem {
   int64_t launches = 0;
   ~pda_problem() {
     if (stepGraph) cudaGraphExecDestroy(stepGraph);
+    if (stepsGraph) cudaGraphExecDestroy(stepsGraph);
     if (hostGraph) cudaGraphExecDestroy(hostGraph);
     if (side) cudaStreamDestroy(side);
     if (evFork) cudaEventDestroy(evFork);

@@ -98,6 +98,20 @@ struct LspgFlags {
   double maxRes;    // max over steps of the residual norm at the step's last iterate
 };
 
+// What becomes of the velocity v of an evaluation (entry q): stored (kind -1),
+// or the explicit stage that consumes it, with the association of the
+// stand-alone update kernels (util.cu),
+//   kind 0: out = x + cb v
+//   kind 1: out = ca y + cb x + cc v
+// so that a stage needs no velocity buffer and no launch of its own.  out is
+// not the evaluated state; it may be y.
+struct StageArgs {
+  int kind = -1;
+  double *out = nullptr;
+  const double *x = nullptr, *y = nullptr;
+  double ca = 0., cb = 0., cc = 0.;
+};
+
 // blocks per reduction group of the fused LSPG kernel's partial sums
 constexpr int kLspgGroup = 16;
 __host__ __device__ constexpr int lspg_groups(int nblocks) { return (nblocks + kLspgGroup - 1) / kLspgGroup; }
