@@ -82,6 +82,15 @@ k_decode_hidden(int h2, const float *__restrict__ W1, const float *__restrict__ 
   __shared__ float sh1[H1];
   __shared__ float sT1[H1][K + 1];  // odd row length: lanes j, j+1 hit different banks
   __shared__ float sx[K];
+  // the row of W2 and the layer-1 weights do not depend on x: in flight first
+  const int lane = threadIdx.x & 31;
+  const int r2 = blockIdx.x * kHiddenWarps + (threadIdx.x >> 5);
+  float wv[H1 / 32];
+  if (r2 < h2) {
+    const float *__restrict__ w = W2 + (long)r2 * H1;
+#pragma unroll
+    for (int i = 0; i < H1 / 32; ++i) wv[i] = __ldg(w + lane + 32 * i);
+  }
   if (threadIdx.x < K) sx[threadIdx.x] = (float)x[threadIdx.x];
   __syncthreads();
   for (int r = threadIdx.x; r < H1; r += blockDim.x) {
@@ -94,13 +103,8 @@ k_decode_hidden(int h2, const float *__restrict__ W1, const float *__restrict__ 
     for (int c = 0; c < K; ++c) sT1[r][c] = d * W1[r * K + c];
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * kHiddenWarps + (threadIdx.x >> 5);
+  const int r = r2;
   if (r >= h2) return;
-  const float *__restrict__ w = W2 + (long)r * H1;
-  float wv[H1 / 32];
-#pragma unroll
-  for (int i = 0; i < H1 / 32; ++i) wv[i] = __ldg(w + lane + 32 * i);  // all loads in flight together
   float acc[ld];
 #pragma unroll
   for (int c = 0; c < ld; ++c) acc[c] = 0.f;
