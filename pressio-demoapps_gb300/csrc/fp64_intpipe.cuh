@@ -130,17 +130,19 @@ __device__ __forceinline__ Den den_prep(double b) {
   return D;
 }
 
-// quotients outside the fast path
-static __device__ __noinline__ double quot_special(double a, double b) { return a / b; }
+// results outside the fast path: zero dividends, and the ordinary division
+static __device__ __noinline__ double quot_special(double a, double b) {
+  const uint64_t ua = (uint64_t)__double_as_longlong(a), ub = (uint64_t)__double_as_longlong(b);
+  const uint32_t eb = (uint32_t)(ub >> 52) & 0x7FFu;
+  if ((ua << 1) == 0 && eb - 1u < 0x7FEu)  // +-0 / normal
+    return __longlong_as_double((long long)((ua ^ ub) & 0x8000000000000000ull));
+  return a / b;
+}
 
 // RN(a / b) for a prepared divisor
 __device__ __forceinline__ double quot(double a, const Den &D) {
   const uint32_t h = hi_word(a), l = lo_word(a);
-  if ((exp_window(h) | D.w) >= (1u << 30)) {
-    // a zero dividend (gas at rest, walls), here: the call below is far away code
-    if ((h << 1 | l) == 0 && D.w < (1u << 30)) return from_words((h ^ hi_word(D.b)) & 0x80000000u, 0u);
-    return quot_special(a, D.b);
-  }
+  if ((exp_window(h) | D.w) >= (1u << 30)) return quot_special(a, D.b);
   const uint64_t ma = (uint64_t)mant_hi(h) << 32 | l;
   const bool ge = ma >= D.mb;
   // sign and (biased exponent - 1): the mantissa's leading bit, and a carry, add one
@@ -176,13 +178,17 @@ __device__ __forceinline__ float rsqrt_seed_f32(float x) {
   return r;
 }
 
-static __device__ __noinline__ double sqrt_special(double x) { return ::sqrt(x); }
+static __device__ __noinline__ double sqrt_special(double x) {
+  const uint64_t ux = (uint64_t)__double_as_longlong(x);
+  if ((ux << 1) == 0) return x;  // +-0
+  return ::sqrt(x);
+}
 
 // RN(sqrt(x))
 __device__ __forceinline__ double sqrt(double x) {
   const uint64_t ux = (uint64_t)__double_as_longlong(x);
   const uint32_t ex = (uint32_t)(ux >> 52);
-  if (ex - 1u >= 0x7FEu) return (ux << 1) == 0 ? x : sqrt_special(x);  // +-0; subnormal, infinite, NaN, negative
+  if (ex - 1u >= 0x7FEu) return sqrt_special(x);  // zero, subnormal, infinite, NaN, negative
   const uint32_t odd = (ex & 1u) ^ 1u;            // parity of ex - 1023
   const uint64_t m = mant53(ux) << odd;           // m 2^-52 in [1, 4)
   const uint32_t mh = (uint32_t)(m >> 22);        // with 30 fraction bits, truncated
