@@ -122,12 +122,12 @@ void rows_vj_inner(int scheme, const RowTable &t, const MeshArgs &m, const Phys 
   switch (scheme) {
     case FirstOrder: k_rows_vj_inner<FAM, FirstOrder><<<g, 64, 0, s>>>(t, m, p, U, rowptr, V, J); break;
     case Weno3: {
-      using RP = RowPar<FAM, Weno3>;
+      using RP = RowPar<FAM>;
       k_rows_vj_inner_par<FAM, Weno3><<<div_up(t.nrows, RP::RPB), RP::THREADS, 0, s>>>(t, m, p, U, rowptr, V, J);
       break;
     }
     default: {
-      using RP = RowPar<FAM, Weno5>;
+      using RP = RowPar<FAM>;
       k_rows_vj_inner_par<FAM, Weno5><<<div_up(t.nrows, RP::RPB), RP::THREADS, 0, s>>>(t, m, p, U, rowptr, V, J);
       break;
     }

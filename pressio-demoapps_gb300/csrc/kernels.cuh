@@ -150,11 +150,11 @@ template <> struct Fam<Swe2d> {
   static constexpr double jac_scale = 1.;
   template <int AXIS, class M, class S>
   static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
-    double JL[ndpc * ndpc], JR[ndpc * ndpc];
+    double J[ndpc * ndpc];
     if (which == 0) flux<AXIS>(fl, qL, qR, p);
-    flux_jac<AXIS>(JL, JR, qL, qR, p);
+    swe_flux_jac_side(J, which, qL, qR, p.gravity, AXIS);
     for (int i = 0; i < ndpc; ++i)
-      for (int j = 0; j < ndpc; ++j) set(i, j, which == 0 ? JL[i * ndpc + j] : JR[i * ndpc + j]);
+      for (int j = 0; j < ndpc; ++j) set(i, j, J[i * ndpc + j]);
   }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<3>;
@@ -244,19 +244,31 @@ PDA_HD double face_value_side(int side, const double *q) {
   }
 }
 
-template <int SCHEME, class M = FpMul, typename T>
-PDA_HD void face_grad_side(int side, T &u, T g[2 * SchemeTraits<SCHEME>::h], const T *q) {
+template <int SCHEME, class M = FpMul, typename T, class Out = NoHandOver>
+PDA_HD void face_grad_side(int side, T &u, T g[2 * SchemeTraits<SCHEME>::h], const T *q, const Out &out = Out{}) {
   if constexpr (SCHEME == FirstOrder) {
     u = q[side];
+    out(u);
     g[0] = side == 0 ? T(1) : T(0);
     g[1] = side == 0 ? T(0) : T(1);
   } else if constexpr (SCHEME == Weno3) {
-    if (side == 0) weno3_neg_grad(u, g, q[0], q[1], q[2], q[3]);
-    else weno3_pos_grad(u, g, q[0], q[1], q[2], q[3]);
+    if (side == 0) weno3_neg_grad(u, g, q[0], q[1], q[2], q[3], out);
+    else weno3_pos_grad(u, g, q[0], q[1], q[2], q[3], out);
   } else {
-    if (side == 0) weno5_neg_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5]);
-    else weno5_pos_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5]);
+    if (side == 0) weno5_neg_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5], out);
+    else weno5_pos_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5], out);
   }
+}
+
+// One-way hand-over inside a block by a named barrier (not 0, __syncthreads's):
+// `threads` counts those that arrive and those that wait, whole warps both.
+template <int ID> __device__ __forceinline__ void bar_arrive(int threads) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(threads) : "memory");
+}
+template <int ID> __device__ __forceinline__ void bar_wait(int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(threads) : "memory");
 }
 
 template <int NDPC>
@@ -578,13 +590,26 @@ k_rows_vj_inner(RowTable t, MeshArgs m, Phys p, const double *__restrict__ U,
 //   phase 1a  thread (side, row, face, dof): one side of the face's
 //             reconstruction (value and, for inner rows, its gradient); the
 //             side is uniform per warp, so each warp evaluates one side only
-//   phase 1b  thread (part, row, face): the face flux (part 0) or the flux
-//             Jacobians (part 1), again one part per warp
-//   phase 2   thread (row, k, j): dof k of V (j == 0) and column dof j of row
-//             k of the row's J blocks, every entry accumulated in exactly the
-//             order of the per-row kernels (k_rows_vj_inner /
-//             k_rows_vj_nearbd), then written once.
+//   phase 1b  thread (part, row, face): the face flux (part 0), the flux
+//             Jacobian with respect to the left or right state (parts 1, 2),
+//             the rows' indices and source terms (part 3), one part per warp;
+//             these warps wait for the values only and run beside 1a's
+//             gradients
+//   phase 2   thread (column block, row, k, j): one entry of the row's J
+//             blocks, accumulated in exactly the order of the per-row kernels
+//             (k_rows_vj_inner / k_rows_vj_nearbd), then written.  Rows of
+//             tiny periodic meshes, some of whose neighbours are the same
+//             cell, take a thread per (row, k, j) that goes through the
+//             blocks in order.
 // Bit-identical to those kernels.
+//
+// 628 shallow-water WENO5 rows: a block's chain went from 47,000 cycles (18,400
+// in 1a, then 17,500 in 1b with both Jacobians in one warp, 10,000 in phase 2
+// in two warps) to 35,000 (values handed over after 8,200, 1b done at 27,000
+// beside the gradients, 4,500 for phase 2), the call 36.9 -> 20.5 us.  Rows per
+// block fill phase 1a's warps: with one row more than the four of before that
+// case's grid is also within one wave (157 -> 126 blocks; 24.6 us by that and
+// the thread per entry alone).
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr int pad_warp(int n) { return (n + 31) / 32 * 32; }
 
@@ -596,125 +621,177 @@ template <int FAM, int SCHEME> struct RowFace {
   double uN[NDPC], uP[NDPC];
 };
 
-template <int FAM, int SCHEME> struct RowPar {
+template <int FAM> struct RowPar {
   static constexpr int NF = 2 * Fam<FAM>::dim, NDPC = Fam<FAM>::ndpc;
-  static constexpr int RPB = 4;                        // rows per block
+  static constexpr int RPB = Fam<FAM>::dim == 3 ? 4 : 64 / (NF * NDPC);  // rows per block
   static constexpr int SIDE = pad_warp(RPB * NF * NDPC);  // phase-1a threads per side
   static constexpr int PART = pad_warp(RPB * NF);         // phase-1b threads per part
-  static constexpr int THREADS = 2 * SIDE;
-  static_assert(2 * PART <= THREADS, "phase 1b fits the block");
+  static constexpr int THREADS = 2 * SIDE + 4 * PART;     // phases 1a and 1b side by side
+  static_assert(PART == 32 && RPB * NDPC <= 32, "a warp covers the block's faces and rows");
 };
 
+// the row's source term (shallow water: Coriolis, swe_2d_prob_class.hpp:
+// 983-1012): its two parts of V, then its Jacobian's entries (1,0), (1,2),
+// (2,1), (2,0); one quotient per thread
+constexpr int kRowSource = 6;
+__device__ __forceinline__ double row_source(int i, const double *q, const Phys &p) {
+  const double c = i == 3 || i == 5 ? -p.coriolis : p.coriolis;
+  const double x = i == 0 || i == 2 ? q[2] : q[1];
+  const double num = i == 3 || i == 4 ? c : c * x;
+  return div_rn(num, i == 2 || i == 5 ? q[0] * q[0] : q[0]);
+}
+
 template <int FAM, int SCHEME>
-__global__ void __launch_bounds__(RowPar<FAM, SCHEME>::THREADS)
+__global__ void __launch_bounds__(RowPar<FAM>::THREADS)
 k_rows_vj_inner_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ U, const int *__restrict__ rowptr,
                     double *__restrict__ V, double *__restrict__ J) {
   using F = Fam<FAM>;
   using RF = RowFace<FAM, SCHEME>;
-  using RP = RowPar<FAM, SCHEME>;
+  using RP = RowPar<FAM>;
   constexpr int NDPC = F::ndpc, DIM = F::dim, H = SchemeTraits<SCHEME>::h, S = 2 * H + 1, G = 2 * H;
   constexpr int NF = RP::NF, RPB = RP::RPB;
   constexpr int NB = 1 + 2 * DIM * H;  // distinct column blocks of an inner row at most
   __shared__ RF fd[RPB][NF];
-  const int tid = threadIdx.x;
-  {  // phase 1a
-    const int side = tid / RP::SIDE, slot = tid % RP::SIDE;
+  __shared__ int sRow[RPB], sBase[RPB][NDPC], sNb[RPB];
+  __shared__ unsigned char sBlk[RPB][DIM][S];
+  __shared__ double sSrc[RPB][kRowSource];
+  const int tid = threadIdx.x, e0 = blockIdx.x * RPB;
+  const int nr = min(RPB, t.nrows - e0);
+  if (tid < 2 * RP::SIDE) {  // phase 1a
+    const int side = tid / RP::SIDE;
+    const bool on = tid % RP::SIDE < nr * NF * NDPC;  // (the other lanes repeat the first)
+    const int slot = on ? tid % RP::SIDE : 0;
     const int rl = slot / (NF * NDPC), f = (slot / NDPC) % NF, d = slot % NDPC, ax = f >> 1, fs = f & 1;
-    const int e = blockIdx.x * RPB + rl;
-    if (slot < RPB * NF * NDPC && e < t.nrows) {
-      double q[G];
-      const size_t base = ((size_t)e * DIM + ax) * S;
+    double q[G];
+    const size_t base = ((size_t)(e0 + rl) * DIM + ax) * S;
 #pragma unroll
-      for (int s = 0; s < G; ++s) q[s] = __ldg(U + (size_t)t.src[base + fs + s] * NDPC + d);
-      RF &o = fd[rl][f];
-      double u, g[G];
-      face_grad_side<SCHEME>(side, u, g, q);
-      double *gs = side == 0 ? o.gN[d] : o.gP[d];
-      (side == 0 ? o.uN : o.uP)[d] = u;
+    for (int s = 0; s < G; ++s) q[s] = __ldg(U + (size_t)t.src[base + fs + s] * NDPC + d);
+    RF &o = fd[rl][f];
+    double u, g[G];
+    face_grad_side<SCHEME>(side, u, g, q, [&](double v) {
+      if (on) (side == 0 ? o.uN : o.uP)[d] = v;
+      bar_arrive<1>(RP::THREADS);
+    });
+    double *gs = side == 0 ? o.gN[d] : o.gP[d];
 #pragma unroll
-      for (int s = 0; s < G; ++s) gs[s] = g[s];
-    }
-  }
-  __syncthreads();
-  {  // phase 1b
-    const int part = tid / RP::PART, slot = tid % RP::PART;
+    for (int s = 0; s < G; ++s)
+      if (on) gs[s] = g[s];
+  } else {  // phase 1b
+    const int part = (tid - 2 * RP::SIDE) / RP::PART, slot = tid % RP::PART;
     const int rl = slot / NF, f = slot % NF, ax = f >> 1;
-    const int e = blockIdx.x * RPB + rl;
-    if (part < 2 && slot < RPB * NF && e < t.nrows) {
+    if (part < 3) bar_wait<1>(RP::THREADS);
+    else bar_arrive<1>(RP::THREADS);
+    if (part < 3 && slot < nr * NF) {
       RF &o = fd[rl][f];
-      double uN[NDPC], uP[NDPC];
+      double uN[NDPC], uP[NDPC], J2[NDPC * NDPC];
 #pragma unroll
       for (int d = 0; d < NDPC; ++d) {
         uN[d] = o.uN[d];
         uP[d] = o.uP[d];
       }
-      if (part == 0) {
-        flux_ax<FAM>(o.fl, uN, uP, p, ax);  // one stream for all axes of the warp
-      } else {
-        F::flux_jac_ax(o.JN, o.JP, uN, uP, p, ax);  // one stream for all axes of the warp
+      // (one stream for all axes of the warp; a Jacobian that is not stored is not computed)
+      if (part == 0) flux_ax<FAM>(o.fl, uN, uP, p, ax);
+      else if (part == 1) F::flux_jac_ax(o.JN, J2, uN, uP, p, ax);
+      else F::flux_jac_ax(J2, o.JP, uN, uP, p, ax);
+    } else if (part == 3) {
+      if (slot < nr * NDPC) {
+        const int rk = slot / NDPC, k = slot % NDPC, r = t.rows[e0 + rk];
+        const int rb = rowptr[r * NDPC + k];
+        sBase[rk][k] = rb;
+        if (k == 0) {
+          sRow[rk] = r;
+          sNb[rk] = (rowptr[r * NDPC + 1] - rb) / NDPC;
+        }
+      }
+      for (int i = slot; i < nr * DIM * S; i += RP::PART)
+        (&sBlk[0][0][0])[i] = (unsigned char)(t.jpos[(size_t)e0 * DIM * S + i] / NDPC);
+      if constexpr (FAM == Swe2d) {
+        for (int i = slot; i < nr * kRowSource; i += RP::PART) {
+          double q[NDPC];
+          load_cell<NDPC>(q, U, t.cell[e0 + i / kRowSource], false, -1);
+          sSrc[i / kRowSource][i % kRowSource] = row_source(i % kRowSource, q, p);
+        }
       }
     }
   }
   __syncthreads();
-  // phase 2: thread (row, k, j)
-  for (int w = tid; w < RPB * NDPC * NDPC; w += blockDim.x) {
+  // phase 2: dof k of the rows' V (last warp)
+  if (tid >= RP::THREADS - 32 && tid - (RP::THREADS - 32) < nr * NDPC) {
+    const int rl = (tid - (RP::THREADS - 32)) / NDPC, k = (tid - (RP::THREADS - 32)) % NDPC;
+    double vk = 0.;
+#pragma unroll
+    for (int ax = 0; ax < DIM; ++ax) vk += m.hinv[ax] * (fd[rl][2 * ax].fl[k] - fd[rl][2 * ax + 1].fl[k]);
+    if constexpr (FAM == Swe2d) {
+      if (k == 1) vk -= sSrc[rl][0];
+      if (k == 2) vk += sSrc[rl][1];
+    }
+    V[(size_t)sRow[rl] * NDPC + k] = vk;
+  }
+  auto source_entry = [&](double &a, int rl, int k, int j) {
+    if constexpr (FAM == Swe2d) {
+      const int i = k == 1 ? (j == 0 ? 2 : j == 2 ? 3 : -1) : k == 2 ? (j == 1 ? 4 : j == 0 ? 5 : -1) : -1;
+      if (i >= 0) a += sSrc[rl][i];
+    }
+  };
+  // entries of the rows' blocks: the cell's own block first (the longest sums), then by axis and position
+  constexpr int RB = RPB * NDPC * NDPC;
+  for (int w = tid; w < NB * RB; w += RP::THREADS) {
+    const int b = w / RB, rl = (w % RB) / (NDPC * NDPC), k = (w / NDPC) % NDPC, j = w % NDPC;
+    if (rl >= nr || sNb[rl] != NB) continue;
+    const int a0 = b == 0 ? 0 : (b - 1) / G, i = b == 0 ? H : (b - 1) % G, pos = b == 0 || i < H ? i : i + 1;
+    const int kj = k * NDPC + j;
+    double acc = 0.;
+#pragma unroll 1
+    for (int ax = a0; ax < (b == 0 ? DIM : a0 + 1); ++ax) {
+      const double hinv = m.hinv[ax];
+      const RF &L = fd[rl][2 * ax], &R = fd[rl][2 * ax + 1];
+      if (pos < G) {
+        acc += L.JN[kj] * L.gN[j][pos] * hinv;
+        acc += L.JP[kj] * L.gP[j][pos] * hinv;
+      }
+      if (pos > 0) {
+        acc -= R.JN[kj] * R.gN[j][pos - 1] * hinv;
+        acc -= R.JP[kj] * R.gP[j][pos - 1] * hinv;
+      }
+    }
+    if (b == 0) source_entry(acc, rl, k, j);
+    J[sBase[rl][k] + sBlk[rl][a0][pos] * NDPC + j] = acc;
+  }
+  // rows with repeated neighbours: thread (row, k, j)
+  for (int w = tid; w < nr * NDPC * NDPC; w += RP::THREADS) {
     const int rl = w / (NDPC * NDPC), k = (w / NDPC) % NDPC, j = w % NDPC;
-    const int e = blockIdx.x * RPB + rl;
-    if (e >= t.nrows) continue;
-    const int r = t.rows[e];
+    if (sNb[rl] == NB) continue;
     double acc[NB];
 #pragma unroll
     for (int i = 0; i < NB; ++i) acc[i] = 0.;
 #pragma unroll 1
     for (int ax = 0; ax < DIM; ++ax) {
       const double hinv = m.hinv[ax];
-      const size_t base = ((size_t)e * DIM + ax) * S;
-      int blk[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) blk[s] = t.jpos[base + s] / NDPC;
+      const unsigned char *blk = sBlk[rl][ax];
       const RF &L = fd[rl][2 * ax], &R = fd[rl][2 * ax + 1];
       const double ln = L.JN[k * NDPC + j], lp = L.JP[k * NDPC + j];
       const double rn = R.JN[k * NDPC + j], rp = R.JP[k * NDPC + j];
-#pragma unroll
+#pragma unroll 1
       for (int s = 0; s < G; ++s) {
         acc[blk[s]] += ln * L.gN[j][s] * hinv;
         acc[blk[s]] += lp * L.gP[j][s] * hinv;
       }
-#pragma unroll
+#pragma unroll 1
       for (int s = 0; s < G; ++s) {
         acc[blk[s + 1]] -= rn * R.gN[j][s] * hinv;
         acc[blk[s + 1]] -= rp * R.gP[j][s] * hinv;
       }
     }
-    double vk = 0.;
-    if (j == 0) {
-#pragma unroll
-      for (int ax = 0; ax < DIM; ++ax) vk += m.hinv[ax] * (fd[rl][2 * ax].fl[k] - fd[rl][2 * ax + 1].fl[k]);
-    }
-    if constexpr (FAM == Swe2d) {
-      // swe_2d_prob_class.hpp:983-1012
-      const int c = t.cell[e];
-      const double u0 = __ldg(U + (size_t)c * 3), u1 = __ldg(U + (size_t)c * 3 + 1),
-                   u2 = __ldg(U + (size_t)c * 3 + 2);
-      if (j == 0 && k == 1) vk -= div_rn(p.coriolis * u2, u0);
-      if (j == 0 && k == 2) vk += div_rn(p.coriolis * u1, u0);
-      const int self = t.jpos[((size_t)e * DIM + 0) * S + H] / NDPC;
-      if (k == 1 && j == 0) acc[self] += div_rn(p.coriolis * u2, (u0 * u0));
-      if (k == 1 && j == 2) acc[self] += div_rn(-p.coriolis, u0);
-      if (k == 2 && j == 1) acc[self] += div_rn(p.coriolis, u0);
-      if (k == 2 && j == 0) acc[self] += div_rn(-p.coriolis * u1, (u0 * u0));
-    }
-    if (j == 0) V[(size_t)r * NDPC + k] = vk;
-    const int rb = rowptr[r * NDPC + k];
-    const int nb = (rowptr[r * NDPC + k + 1] - rb) / NDPC;
-    for (int b = 0; b < nb && b < NB; ++b) J[rb + b * NDPC + j] = acc[b];
+    source_entry(acc[sBlk[rl][0][H]], rl, k, j);
+    for (int b = 0; b < sNb[rl] && b < NB; ++b) J[sBase[rl][k] + b * NDPC + j] = acc[b];
   }
 }
 
 // Near-boundary rows, split the same way: phase 1a one side of the scheme's
 // face value (ghost entries through their recipes), phase 1b the face flux
-// (part 0) or the first-order flux Jacobians of the face's two cells (part 1),
-// phase 2 thread (row, k, j) accumulates exactly as k_rows_vj_nearbd does.
+// (part 0), the first-order flux Jacobian of the face's left or right cell
+// (parts 1, 2), or the rows' source terms (part 3), phase 2 thread (row, k, j)
+// accumulates exactly as k_rows_vj_nearbd does.
 template <int FAM> struct NearFace {
   static constexpr int NDPC = Fam<FAM>::ndpc;
   double fl[NDPC];
@@ -727,8 +804,7 @@ template <int FAM> struct NearPar {
   static constexpr int RPB = 4;
   static constexpr int SIDE = pad_warp(RPB * NF * NDPC);
   static constexpr int PART = pad_warp(RPB * NF);
-  static constexpr int THREADS = 2 * SIDE;
-  static_assert(2 * PART <= THREADS, "phase 1b fits the block");
+  static constexpr int THREADS = 2 * SIDE > 4 * PART ? 2 * SIDE : 4 * PART;
 };
 
 template <int FAM, int SCHEME>
@@ -740,12 +816,13 @@ k_rows_vj_nearbd_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ 
   constexpr int NDPC = F::ndpc, DIM = F::dim, H = SchemeTraits<SCHEME>::h, S = 2 * H + 1, G = 2 * H;
   constexpr int NF = NP::NF, RPB = NP::RPB, NB = 1 + 2 * DIM;
   __shared__ NearFace<FAM> fd[RPB][NF];
+  __shared__ double sSrc[RPB][kRowSource];
   const int tid = threadIdx.x;
   {  // phase 1a
     const int side = tid / NP::SIDE, slot = tid % NP::SIDE;
     const int rl = slot / (NF * NDPC), f = (slot / NDPC) % NF, d = slot % NDPC, ax = f >> 1, fs = f & 1;
     const int e = blockIdx.x * RPB + rl;
-    if (slot < RPB * NF * NDPC && e < t.nrows) {
+    if (side < 2 && slot < RPB * NF * NDPC && e < t.nrows) {
       double q[G];
       const size_t base = ((size_t)e * DIM + ax) * S;
 #pragma unroll
@@ -763,7 +840,7 @@ k_rows_vj_nearbd_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ 
     const int part = tid / NP::PART, slot = tid % NP::PART;
     const int rl = slot / NF, f = slot % NF, ax = f >> 1, fs = f & 1;
     const int e = blockIdx.x * RPB + rl;
-    if (part < 2 && slot < RPB * NF && e < t.nrows) {
+    if (part < 3 && slot < RPB * NF && e < t.nrows) {
       NearFace<FAM> &o = fd[rl][f];
       if (part == 0) {
         double uN[NDPC], uP[NDPC];
@@ -780,7 +857,20 @@ k_rows_vj_nearbd_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ 
         for (int s = 0; s < 2; ++s)
           load_entry<NDPC>(q1[s], U, t.src1[b1 + fs + s], t.flip1[b1 + fs + s], m.reflect[ax], m, t.gsx1, t.gsy1,
                            b1 + fs + s);
-        F::flux_jac_ax(o.JN, o.JP, q1[0], q1[1], p, ax);  // one stream for all axes of the warp
+        // (one stream for all axes of the warp; the Jacobian that is not stored is not computed)
+        double J2[NDPC * NDPC];
+        if (part == 1) F::flux_jac_ax(o.JN, J2, q1[0], q1[1], p, ax);
+        else F::flux_jac_ax(J2, o.JP, q1[0], q1[1], p, ax);
+      }
+    } else if (part == 3) {
+      if constexpr (FAM == Swe2d) {
+        for (int i = slot; i < RPB * kRowSource; i += NP::PART) {
+          const int es = blockIdx.x * RPB + i / kRowSource;
+          if (es >= t.nrows) break;
+          double q[NDPC];
+          load_cell<NDPC>(q, U, t.cell[es], false, -1);
+          sSrc[i / kRowSource][i % kRowSource] = row_source(i % kRowSource, q, p);
+        }
       }
     }
   }
@@ -816,16 +906,11 @@ k_rows_vj_nearbd_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ 
       for (int ax = 0; ax < DIM; ++ax) vk += m.hinv[ax] * (fd[rl][2 * ax].fl[k] - fd[rl][2 * ax + 1].fl[k]);
     }
     if constexpr (FAM == Swe2d) {
-      const int c = t.cell[e];
-      const double u0 = __ldg(U + (size_t)c * 3), u1 = __ldg(U + (size_t)c * 3 + 1),
-                   u2 = __ldg(U + (size_t)c * 3 + 2);
-      if (j == 0 && k == 1) vk -= div_rn(p.coriolis * u2, u0);
-      if (j == 0 && k == 2) vk += div_rn(p.coriolis * u1, u0);
+      if (j == 0 && k == 1) vk -= sSrc[rl][0];
+      if (j == 0 && k == 2) vk += sSrc[rl][1];
       const int self = t.jpos1[((size_t)e * DIM + 0) * 3 + 1] / 3;
-      if (k == 1 && j == 0) acc[self] += div_rn(p.coriolis * u2, (u0 * u0));
-      if (k == 1 && j == 2) acc[self] += div_rn(-p.coriolis, u0);
-      if (k == 2 && j == 1) acc[self] += div_rn(p.coriolis, u0);
-      if (k == 2 && j == 0) acc[self] += div_rn(-p.coriolis * u1, (u0 * u0));
+      const int i = k == 1 ? (j == 0 ? 2 : j == 2 ? 3 : -1) : k == 2 ? (j == 1 ? 4 : j == 0 ? 5 : -1) : -1;
+      if (i >= 0) acc[self] += sSrc[rl][i];
     }
     if (j == 0) V[(size_t)r * NDPC + k] = vk;
     const int rb = rowptr[r * NDPC + k];

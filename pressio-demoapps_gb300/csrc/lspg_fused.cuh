@@ -22,13 +22,13 @@
 // k_rows_vj_nearbd_par (GB300's narrow FP64 units make the per-thread
 // instruction chain the cost, so the work of a row is spread over threads).
 // An iteration is one wave of blocks and its time one block's chain, not a
-// rate: at 628 shallow-water rows with 12 latents about 45,000 cycles, of which
-// the loads and face values take 12,000, the fluxes 7,000, the columns and the
-// products 10,000, the groups' sums 5,000 and the solve 13,000.  A Gauss-Newton
-// step with its decoder went 51.4 -> 48.6 us with the L D L^T solve and the
-// batched sums, 45.3 with the rows' states and histories on warps of their own,
-// 44.0 with the copies' table entries loaded ahead and the pivots' products
-// beside their reciprocals.
+// rate: at 628 shallow-water rows with 12 latents about 43,000 cycles, of which
+// the loads, face values and fluxes take 17,000, the columns and the products
+// 10,000, the groups' sums 5,000 and the solve 11,000.  A Gauss-Newton step
+// with its decoder went 51.4 -> 48.6 us with the L D L^T solve and the batched
+// sums, 44.8 with the rows' states and histories on warps of their own and the
+// copies' table entries loaded ahead, 43.3 with the fluxes on warps that start
+// when the values are there.
 #pragma once
 
 #include "kernels.cuh"
@@ -45,10 +45,8 @@ template <int FAM> struct FusedPar {
   static constexpr int RPB_MAX = Fam<FAM>::dim == 3 ? 4 : 8;
   static constexpr int SIDE = pad_warp(RPB_MAX * NF * NDPC);
   static constexpr int PART = pad_warp(RPB_MAX * NF);
-  // the two sides of phase A and two warps beside them for the rows' states and histories; with these, phases C
-  // and D of the usual sizes take one round
-  static constexpr int THREADS = 2 * SIDE + 64;
-  static_assert(4 * PART <= THREADS, "phase B fits the block");
+  // phase A's two sides, phase B's four parts, and two warps for the rows' states and histories, side by side
+  static constexpr int THREADS = 2 * SIDE + 4 * PART + 64;
   static_assert(RPB_MAX * NF <= PART && RPB_MAX * NDPC <= 32, "a warp covers the block's faces and rows");
   static constexpr size_t kSmemLimit = 160 * 1024;  // dynamic shared memory per block
   // dynamic shared memory per row: staged D of the row's stencil cells, the
@@ -228,6 +226,7 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
   __shared__ LspgTables tabs;
   __shared__ typename F::Side sSide[FP::RPB_MAX][NF][2];  // the two face states' halves of the flux
   extern __shared__ double dyn[];
+  constexpr int kHandOver = 2 * FP::SIDE + 4 * FP::PART;
   const int tid = threadIdx.x, K = a.K, RD = rpb * NDPC, CB = NDPC * K;  // CB: D doubles per cell
   double *sD = dyn;                                  // [rpb][DIM][S][NDPC][K] staged D of stencil cells
   double *ctb = sD + (size_t)rpb * DIM * S * CB;     // [rpb][NF][NDPC][K]
@@ -287,131 +286,111 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
       sSJ[rl][2 * 3 + 0] = div_rn(-p.coriolis * u1, (u0 * u0));
     }
   };
-  if (tid >= 2 * FP::SIDE + 32) {
-    const int rk = tid - 2 * FP::SIDE - 32, e = e0 + rk / NDPC;
-    if (rk < rpb * NDPC && e < t.nrows) {
-      const int r = t.rows[e];
+  // GB300 issues one FP64 warp instruction per ~64 cycles per sub-partition
+  // whatever the number of active lanes, so the time is the longest per-warp
+  // chain.  Phase A's warps hand the face values over before they go on to the
+  // gradients; phase B's, beside them, form the two face states' halves of the
+  // flux (parts 0, 1, then part 0 their combination) and JN, JP (parts 2, 3).
+  const int nrow = min(rpb, t.nrows - e0);
+  if (tid < 2 * FP::SIDE) {  // phase A: (side, row, face, dof): one side of the face value (+ gradient for inner rows)
+    const int side = tid / FP::SIDE;
+    const bool on = tid % FP::SIDE < nrow * NF * NDPC;  // (the other lanes repeat the first)
+    const int slot = on ? tid % FP::SIDE : 0;
+    const int rl = slot / (NF * NDPC), f = (slot / NDPC) % NF, d = slot % NDPC, ax = f >> 1, fs = f & 1;
+    const size_t base = ((size_t)(e0 + rl) * DIM + ax) * S;
+    double q[G];
+    FF &o = fd[rl][f];
+    auto hand_over = [&](double v) {
+      if (on) (side == 0 ? o.uN : o.uP)[d] = v;
+      bar_arrive<1>(kHandOver);
+    };
+    if (inner) {
+#pragma unroll
+      for (int s = 0; s < G; ++s) q[s] = __ldg(a.y + (size_t)t.src[base + fs + s] * NDPC + d);
+      JT u, gg[G];
+      if constexpr (kExact) {
+        face_grad_side<SCHEME>(side, u, gg, q, hand_over);
+      } else {
+        // the value in double (it enters V and R); the gradient in float
+        hand_over(face_value_side<SCHEME>(side, q));
+        JT qf[G];
+#pragma unroll
+        for (int s = 0; s < G; ++s) qf[s] = (JT)q[s];
+        face_grad_side<SCHEME>(side, u, gg, qf);
+      }
+      JT *gs = side == 0 ? o.gN[d] : o.gP[d];
+#pragma unroll
+      for (int s = 0; s < G; ++s)
+        if (on) gs[s] = gg[s];
+    } else {
+#pragma unroll
+      for (int s = 0; s < G; ++s) {
+        double qe[NDPC];
+        load_entry<NDPC>(qe, a.y, t.src[base + fs + s], t.flip[base + fs + s], m.reflect[ax], m, t.gsx, t.gsy,
+                         base + fs + s);
+        q[s] = qe[d];
+      }
+      hand_over(face_value_side<SCHEME>(side, q));
+    }
+  } else if (tid < 2 * FP::SIDE + 4 * FP::PART) {  // phase B: (part, row, face)
+    const int part = (tid - 2 * FP::SIDE) / FP::PART, slot = (tid - 2 * FP::SIDE) % FP::PART;
+    const int rl = slot / NF, f = slot % NF, ax = f >> 1, fs = f & 1;
+    const bool on = slot < nrow * NF;
+    bar_wait<1>(kHandOver);
+    if (part < 2) {
+      // (one stream for all axes of the warp)
+      if (on) F::flux_side_ax(sSide[rl][f][part], part == 0 ? fd[rl][f].uN : fd[rl][f].uP, p, ax);
+      if (part == 1) bar_arrive<2>(2 * FP::PART);
+      else bar_wait<2>(2 * FP::PART);
+      if (part == 0 && on) {
+        FF &o = fd[rl][f];
+        const typename F::Side &L = sSide[rl][f][0], &R = sSide[rl][f][1];
+        F::template flux_combine<0>(o.fl, o.uN, o.uP, L, R, p);  // the combination does not depend on the axis
+      }
+    } else if (on) {
+      FF &o = fd[rl][f];
+      double uN[NDPC], uP[NDPC];
+#pragma unroll
+      for (int d = 0; d < NDPC; ++d) {
+        uN[d] = o.uN[d];
+        uP[d] = o.uP[d];
+      }
+      if (!inner) {
+        // first-order Jacobian at the face's two cells (ghosts through their recipes)
+        const size_t b1 = ((size_t)(e0 + rl) * DIM + ax) * 3;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          double qe[NDPC];
+          load_entry<NDPC>(qe, a.y, t.src1[b1 + fs + s], t.flip1[b1 + fs + s], m.reflect[ax], m, t.gsx1, t.gsy1,
+                           b1 + fs + s);
+#pragma unroll
+          for (int d = 0; d < NDPC; ++d) (s == 0 ? uN : uP)[d] = qe[d];
+        }
+      }
+      JT J2[NDPC * NDPC], vN[NDPC], vP[NDPC];
+#pragma unroll
+      for (int d = 0; d < NDPC; ++d) {
+        vN[d] = (JT)uN[d];
+        vP[d] = (JT)uP[d];
+      }
+      // (one stream for all axes of the warp; the Jacobian that is not stored is not computed)
+      if (part == 2) F::flux_jac_ax(o.JN, J2, vN, vP, p, ax);
+      else F::flux_jac_ax(J2, o.JP, vN, vP, p, ax);
+    }
+  } else if (tid < 2 * FP::SIDE + 4 * FP::PART + 32) {
+    row_state_and_source(tid - 2 * FP::SIDE - 4 * FP::PART);
+  } else {
+    const int rk = tid - 2 * FP::SIDE - 4 * FP::PART - 32;
+    if (rk < nrow * NDPC) {
+      const int r = t.rows[e0 + rk / NDPC];
       if (rk % NDPC == 0) sRow[rk / NDPC] = r;
       sHist[0][rk] = a.yn[(size_t)r * NDPC + rk % NDPC];
       sHist[1][rk] = a.ynm1[(size_t)r * NDPC + rk % NDPC];
     }
-    lspg_tables(tabs, K, tid - 2 * FP::SIDE - 32, 32);
-  } else if (tid >= 2 * FP::SIDE) {
-    row_state_and_source(tid - 2 * FP::SIDE);
-  }
-  {  // phase A: (side, row, face, dof): one side of the face value (+ gradient for inner rows)
-    const int side = tid / FP::SIDE, slot = tid % FP::SIDE;
-    const int rl = slot / (NF * NDPC), f = (slot / NDPC) % NF, d = slot % NDPC, ax = f >> 1, fs = f & 1;
-    const int e = e0 + rl;
-    if (side < 2 && slot < rpb * NF * NDPC && e < t.nrows) {
-      const size_t base = ((size_t)e * DIM + ax) * S;
-      double q[G];
-      FF &o = fd[rl][f];
-      if (inner) {
-#pragma unroll
-        for (int s = 0; s < G; ++s) q[s] = __ldg(a.y + (size_t)t.src[base + fs + s] * NDPC + d);
-        JT u, gg[G];
-        if constexpr (kExact) {
-          face_grad_side<SCHEME>(side, u, gg, q);
-        } else {
-          // the value in double (it enters V and R); the gradient in float
-          JT qf[G];
-#pragma unroll
-          for (int s = 0; s < G; ++s) qf[s] = (JT)q[s];
-          face_grad_side<SCHEME>(side, u, gg, qf);
-        }
-        JT *gs = side == 0 ? o.gN[d] : o.gP[d];
-        (side == 0 ? o.uN : o.uP)[d] = kExact ? (double)u : face_value_side<SCHEME>(side, q);
-#pragma unroll
-        for (int s = 0; s < G; ++s) gs[s] = gg[s];
-      } else {
-#pragma unroll
-        for (int s = 0; s < G; ++s) {
-          double qe[NDPC];
-          load_entry<NDPC>(qe, a.y, t.src[base + fs + s], t.flip[base + fs + s], m.reflect[ax], m, t.gsx, t.gsy,
-                           base + fs + s);
-          q[s] = qe[d];
-        }
-        (side == 0 ? o.uN : o.uP)[d] = face_value_side<SCHEME>(side, q);
-      }
-    }
+    lspg_tables(tabs, K, rk, 32);
   }
   cp_async_wait_all();
   __syncthreads();
-  // GB300 issues one FP64 warp instruction per ~64 cycles per sub-partition
-  // whatever the number of active lanes, so a stage costs its longest
-  // per-warp FP64 instruction stream.  With single-precision Jacobian terms
-  // phase B runs in two stages so that no warp evaluates a whole flux: B1 the
-  // two face states' halves of the flux (warps 0 / 1) beside JN / JP (warps
-  // 2 / 3), B2 their combination (warp 0).  With double-precision Jacobian
-  // terms the flux Jacobians are the longest streams, so one stage: warp 0 the
-  // whole flux.
-  auto combine = [&](int rl, int f) {
-    FF &o = fd[rl][f];
-    const typename F::Side &L = sSide[rl][f][0], &R = sSide[rl][f][1];
-    F::template flux_combine<0>(o.fl, o.uN, o.uP, L, R, p);  // the combination does not depend on the axis
-  };
-  {  // phase B1: (part, row, face): parts 0 / 1 the left / right face state's
-     // half of the flux (exact Jacobian: part 0 both halves and the flux),
-     // parts 2 / 3 JN / JP
-    const int part = tid / FP::PART, slot = tid % FP::PART;
-    const int rl = slot / NF, f = slot % NF, ax = f >> 1, fs = f & 1;
-    const int e = e0 + rl;
-    if (part < 4 && !(kExact && part == 1) && slot < rpb * NF && e < t.nrows) {
-      FF &o = fd[rl][f];
-      if (part < 2) {
-#pragma unroll
-        for (int sd = 0; sd < (kExact ? 2 : 1); ++sd) {
-          const int side = kExact ? sd : part;
-          const double *q = side == 0 ? o.uN : o.uP;
-          typename F::Side &so = sSide[rl][f][side];
-          F::flux_side_ax(so, q, p, ax);  // one stream for all axes of the warp
-        }
-        if (kExact) combine(rl, f);
-      } else {
-        double uN[NDPC], uP[NDPC];
-#pragma unroll
-        for (int d = 0; d < NDPC; ++d) {
-          uN[d] = o.uN[d];
-          uP[d] = o.uP[d];
-        }
-        if (!inner) {
-          // first-order Jacobian at the face's two cells (ghosts through their recipes)
-          const size_t b1 = ((size_t)e * DIM + ax) * 3;
-#pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            double qe[NDPC];
-            load_entry<NDPC>(qe, a.y, t.src1[b1 + fs + s], t.flip1[b1 + fs + s], m.reflect[ax], m, t.gsx1,
-                             t.gsy1, b1 + fs + s);
-#pragma unroll
-            for (int d = 0; d < NDPC; ++d) (s == 0 ? uN : uP)[d] = qe[d];
-          }
-        }
-        JT JN[NDPC * NDPC], JP[NDPC * NDPC], vN[NDPC], vP[NDPC];
-#pragma unroll
-        for (int d = 0; d < NDPC; ++d) {
-          vN[d] = (JT)uN[d];
-          vP[d] = (JT)uP[d];
-        }
-        F::flux_jac_ax(JN, JP, vN, vP, p, ax);  // one stream for all axes of the warp
-        // one of the two per warp (the part is warp-uniform): the other's
-        // arithmetic is dead and dropped
-        if (part == 2) {
-#pragma unroll
-          for (int i = 0; i < NDPC * NDPC; ++i) o.JN[i] = JN[i];
-        } else {
-#pragma unroll
-          for (int i = 0; i < NDPC * NDPC; ++i) o.JP[i] = JP[i];
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if constexpr (!kExact) {  // phase B2: (row, face) the flux from its two halves
-    const int rl = tid / NF, f = tid % NF;
-    if (tid < rpb * NF && e0 + rl < t.nrows) combine(rl, f);
-    __syncthreads();
-  }
   // phase C: (row, face, column c): the face's (JN dU_N + JP dU_P) D column
   for (int w = tid; w < rpb * NF * K; w += blockDim.x) {
     const int rl = w / (NF * K), f = (w / K) % NF, c = w % K, ax = f >> 1, fs = f & 1;

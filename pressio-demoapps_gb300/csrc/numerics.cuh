@@ -27,6 +27,8 @@
 
 #include <math.h>
 
+#include <type_traits>
+
 #include "fp64_intpipe.cuh"
 
 #if defined(__CUDACC__)
@@ -335,6 +337,12 @@ struct IpMul {
   static PDA_HD double mul(double x, double y) { return mul_ip_out(x, y); }
 };
 
+// What a gradient routine does with its face value, before the gradient itself:
+// nothing, or (row kernels) hand it to the warps that form the flux.
+struct NoHandOver {
+  template <typename T> PDA_HD void operator()(T) const {}
+};
+
 // whether x is infinite or NaN, from its bits on the device
 PDA_HD bool not_finite(double x) {
 #if defined(__CUDA_ARCH__)
@@ -343,6 +351,7 @@ PDA_HD bool not_finite(double x) {
   return !(x - x == 0.);
 #endif
 }
+PDA_HD bool not_finite(float x) { return !(x - x == 0.f); }
 // x^3 from x and p = x^2 (see cube)
 template <class M>
 PDA_HD double cube_of(double x, double p) {
@@ -366,25 +375,38 @@ PDA_HD float cube_of(float x, float p) { return p * x; }
 // cS below, and so every component is NaN, as there), and a factor of -2 is
 // exact, so it joins the next sum: 94 FP64 instructions where the full loops
 // take 124.
-template <class M, typename T>
+template <class M, typename T, class Out>
 PDA_HD void weno5_side_grad(T &u, T *g, const T p[3], const T B[3], const T na[3], const T d0[3], const T d1[3],
-                            const T d2[3], const T t[9]) {
+                            const T d2[3], const T t[9], const Out &out) {
   constexpr T epsilon = T(1e-6);
-  T al[3], c[3];
+  // (a value handed over comes first; else all six quotients stand together, with fewer values alive: the Jacobian
+  // tile's kernel, 512^2, 1863 us so, 2061 the other way)
+  constexpr bool early = !std::is_same<Out, NoHandOver>::value;
+  T al[3], c[3], e[3], s[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const T e = B[k] + epsilon;
-    const T s = M::mul(e, e);
-    al[k] = div_rn(na[k] / T(10.), s);
-    c[k] = div_rn(-na[k], T(5.) * cube_of<M>(e, s));
+    e[k] = B[k] + epsilon;
+    s[k] = M::mul(e[k], e[k]);
+    al[k] = div_rn(na[k] / T(10.), s[k]);
+    if (!early) c[k] = div_rn(-na[k], T(5.) * cube_of<M>(e[k], s[k]));
   }
   const T aS = div_rn(T(1.), (al[0] + al[1] + al[2]));
+  T w0, w1, w2;
+  auto value = [&] {
+    w0 = M::mul(al[0], aS), w1 = M::mul(al[1], aS), w2 = M::mul(al[2], aS);
+    u = M::mul(w0, p[0]) + M::mul(w1, p[1]) + M::mul(w2, p[2]);
+    out(u);
+  };
+  if (early) {
+    value();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) c[k] = div_rn(-na[k], T(5.) * cube_of<M>(e[k], s[k]));
+  }
   const T sr = al[2] + al[1] + al[0];
   T cS = div_rn(-T(1.), M::mul(sr, sr));
   if (sizeof(T) == 8 && (not_finite((double)c[0]) || not_finite((double)c[1]) || not_finite((double)c[2])))
     cS = c[0] + c[1] + c[2] + (c[0] - c[0]) + (c[1] - c[1]) + (c[2] - c[2]);  // NaN
-  const T w0 = M::mul(al[0], aS), w1 = M::mul(al[1], aS), w2 = M::mul(al[2], aS);
-  u = M::mul(w0, p[0]) + M::mul(w1, p[1]) + M::mul(w2, p[2]);
+  if (!early) value();
   // da0 = {x0, -2 x1, x2}, da1 = {y0, -2 y1, y2}, da2 = {z0, -2 z1, z2}
   const T x0 = M::mul(c[0], d0[0]), x1 = M::mul(c[0], d0[1]), x2 = M::mul(c[0], d0[2]);
   const T y0 = M::mul(c[1], d1[0]), y1 = M::mul(c[1], d1[1]), y2 = M::mul(c[1], d1[2]);
@@ -451,8 +473,8 @@ PDA_HD T w5_indicator(T X, T Y) {
 // WENO5 with the gradient of the two face values with respect to the six
 // stencil values q_{i-2..i+3}: gNeg[5] == 0, gPos[0] == 0.
 // one side of weno5_face_grad: uNeg and its gradient
-template <class M = FpMul, typename T>
-PDA_HD void weno5_neg_grad(T &uNeg, T gNeg[6], T qim2, T qim1, T qi, T qip1, T qip2, T qip3) {
+template <class M = FpMul, typename T, class Out = NoHandOver>
+PDA_HD void weno5_neg_grad(T &uNeg, T gNeg[6], T qim2, T qim1, T qi, T qip1, T qip2, T qip3, const Out &out = Out{}) {
   constexpr T oneOvsix = T(1.) / T(6.);
   const T na[3] = {T(1.), T(6.), T(3.)};
   const T t[9] = {T(1.) / T(3.),  -T(7.) / T(6.), T(11.) / T(6.), -T(1.) / T(6.), T(5.) / T(6.),
@@ -466,13 +488,13 @@ PDA_HD void weno5_neg_grad(T &uNeg, T gNeg[6], T qim2, T qim1, T qi, T qip1, T q
   w5_outer_derivs(d0[0], d0[1], d0[2], T(13.) * C0, Y0);
   w5_mid_derivs(d1[0], d1[1], d1[2], T(13.) * fma_p2(-T(2.), qi, qip1 + qim1), Y1);
   w5_outer_derivs(d2[2], d2[1], d2[0], T(13.) * w5_curv(qip2, qip1, qi), w5_slopeL(qip2, qip1, qi));
-  weno5_side_grad<M>(uNeg, gNeg, p, B, na, d0, d1, d2, t);
+  weno5_side_grad<M>(uNeg, gNeg, p, B, na, d0, d1, d2, t, out);
   gNeg[5] = T(0.);
 }
 
 // one side of weno5_face_grad: uPos and its gradient
-template <class M = FpMul, typename T>
-PDA_HD void weno5_pos_grad(T &uPos, T gPos[6], T qim2, T qim1, T qi, T qip1, T qip2, T qip3) {
+template <class M = FpMul, typename T, class Out = NoHandOver>
+PDA_HD void weno5_pos_grad(T &uPos, T gPos[6], T qim2, T qim1, T qi, T qip1, T qip2, T qip3, const Out &out = Out{}) {
   constexpr T oneOvsix = T(1.) / T(6.);
   const T na[3] = {T(3.), T(6.), T(1.)};
   const T t[9] = {-T(1.) / T(6.), T(5.) / T(6.),  T(1.) / T(3.),  T(1.) / T(3.), T(5.) / T(6.),
@@ -488,7 +510,7 @@ PDA_HD void weno5_pos_grad(T &uPos, T gPos[6], T qim2, T qim1, T qi, T qip1, T q
                   fma_p2(-T(4.), qi, T(3.) * qip1 + qim1));
   w5_mid_derivs(d1[0], d1[1], d1[2], T(13.) * w5_curv(qip2, qip1, qi), Y1);
   w5_outer_derivs(d2[2], d2[1], d2[0], T(13.) * w5_curv(qip3, qip2, qip1), w5_slopeL(qip3, qip2, qip1));
-  weno5_side_grad<M>(uPos, gPos + 1, p, B, na, d0, d1, d2, t);
+  weno5_side_grad<M>(uPos, gPos + 1, p, B, na, d0, d1, d2, t, out);
   gPos[0] = T(0.);
 }
 
@@ -552,8 +574,8 @@ PDA_HD void weno3_face(double &uNeg, double &uPos, double qim1, double qi,
 
 // WENO3 with gradients with respect to q_{i-1..i+2}: gNeg[3] == 0, gPos[0] == 0.
 // one side of weno3_face_grad: uNeg and its gradient
-template <typename T>
-PDA_HD void weno3_neg_grad(T &uNeg, T gNeg[4], T qim1, T qi, T qip1, T qip2) {
+template <typename T, class Out = NoHandOver>
+PDA_HD void weno3_neg_grad(T &uNeg, T gNeg[4], T qim1, T qi, T qip1, T qip2, const Out &out = Out{}) {
   constexpr T epsilon = T(1e-6);
   constexpr T two = T(2.), three = T(3.);
   constexpr T oneOvtwo = T(1.) / T(2.), oneOvthree = T(1.) / T(3.), twoOvthree = T(2.) / T(3.);
@@ -567,6 +589,10 @@ PDA_HD void weno3_neg_grad(T &uNeg, T gNeg[4], T qim1, T qi, T qip1, T qip2) {
     const T alpha0 = div_rn(oneOvthree, (epsilon * epsilon + two * epsilon * B0 + B0 * B0));
     const T alpha1 = div_rn(twoOvthree, (epsilon * epsilon + two * epsilon * B1 + B1 * B1));
     const T alphaSInv = div_rn(T(1.), (alpha0 + alpha1));
+    const T w0 = alpha0 * alphaSInv;
+    const T w1 = alpha1 * alphaSInv;
+    uNeg = w0 * p0 + w1 * p1;
+    out(uNeg);
     const T e0 = sq(qim1 - qi) + epsilon;  // pow(pow(qim1-qi,2.)+eps, .)
     const T e1 = sq(qi - qip1) + epsilon;
     const T A = div_rn(T(2.), (T(3.) * sq(e1))) + div_rn(T(1.), (T(3.) * sq(e0)));
@@ -580,21 +606,18 @@ PDA_HD void weno3_neg_grad(T &uNeg, T gNeg[4], T qim1, T qi, T qip1, T qip2) {
     daS[0] = div_rn((T(4.) * (qim1 - qi)), (T(3.) * cube(e0) * sq(A)));
     daS[1] = div_rn(-(div_rn((T(4.) * (qim1 - qi)), (T(3.) * cube(e0))) - div_rn((T(8.) * (qi - qip1)), (T(3.) * cube(e1)))), sq(A));
     daS[2] = div_rn(-(T(8.) * (qi - qip1)), (T(3.) * sq(A) * cube(e1)));
-    const T w0 = alpha0 * alphaSInv;
-    const T w1 = alpha1 * alphaSInv;
     for (int i = 0; i < 3; i++) {
       T g = (da0[i] * alphaSInv + daS[i] * alpha0) * p0 + dp0[i] * w0;
       g += (da1[i] * alphaSInv + daS[i] * alpha1) * p1 + dp1[i] * w1;
       gNeg[i] = g;
     }
     gNeg[3] = T(0.);
-    uNeg = w0 * p0 + w1 * p1;
   }
 }
 
 // one side of weno3_face_grad: uPos and its gradient
-template <typename T>
-PDA_HD void weno3_pos_grad(T &uPos, T gPos[4], T qim1, T qi, T qip1, T qip2) {
+template <typename T, class Out = NoHandOver>
+PDA_HD void weno3_pos_grad(T &uPos, T gPos[4], T qim1, T qi, T qip1, T qip2, const Out &out = Out{}) {
   constexpr T epsilon = T(1e-6);
   constexpr T two = T(2.), three = T(3.);
   constexpr T oneOvtwo = T(1.) / T(2.), oneOvthree = T(1.) / T(3.), twoOvthree = T(2.) / T(3.);
@@ -608,6 +631,8 @@ PDA_HD void weno3_pos_grad(T &uPos, T gPos[4], T qim1, T qi, T qip1, T qip2) {
     const T alphaSInv = div_rn(T(1.), (alpha0 + alpha1));
     const T w0 = alpha0 * alphaSInv;
     const T w1 = alpha1 * alphaSInv;
+    uPos = w0 * p0 + w1 * p1;
+    out(uPos);
     const T dp0[3] = {T(1.) / T(2.), 1 / T(2.), T(0.)};
     const T dp1[3] = {T(0.), T(3.) / T(2.), -T(1.) / T(2.)};
     const T e0 = sq(qi - qip1) + epsilon;
@@ -629,7 +654,6 @@ PDA_HD void weno3_pos_grad(T &uPos, T gPos[4], T qim1, T qi, T qip1, T qip2) {
       gPos[i + 1] = g;
     }
     gPos[0] = T(0.);
-    uPos = w0 * p0 + w1 * p1;
   }
 }
 
@@ -1311,59 +1335,68 @@ PDA_HD void euler_flux_jac2(int which, double *fl, S set, const double *qL, cons
     }
 }
 
-// Shallow-water Rusanov flux Jacobian (generic normal).  deviation: pow(x,0.5)
-// -> sqrt(x); pow(2,3/2) is the correctly rounded constant 2*sqrt(2).
+// Shallow-water Rusanov flux Jacobian with respect to the left (side 0) or the
+// right state; u_n, q_n and u_t, q_t are the normal's and the other component.
+// Products with the normal's 0 and 1 are left out: a zero factor's term is zero
+// unless a value is not finite, and then, as in the full form, hsum (hence dn,
+// dt and every entry) is NaN; the exact halves of a sum's terms are taken once,
+// of the sum.  One face costs 45 FP64 instructions and 13 divisions and roots
+// a side where the generic form takes 100 and 19.
+// deviation: pow(x,0.5) -> sqrt(x); pow(2,3/2) is the correctly rounded
+// constant 2*sqrt(2).
 template <typename T>
-PDA_HD void swe_flux_jac_ax(T JL[9], T JR[9], const T qL[3],
-                         const T qR[3], T g, int ax) {
+PDA_HD void swe_flux_jac_side(T J[9], int side, const T qL[3], const T qR[3], T g, int ax) {
   constexpr T es = T(1.e-30);
-  const T n[2] = {ax == 0 ? T(1.) : T(0.), ax == 1 ? T(1.) : T(0.)};
-  const T hL = qL[0];
-  const T uL = div_rn(qL[1], (hL + es));
-  const T vL = div_rn(qL[2], (hL + es));
-  const T unL = uL * n[0] + vL * n[1];
-  const T hR = qR[0];
-  const T uR = div_rn(qR[1], (hR + es));
-  const T vR = div_rn(qR[2], (hR + es));
-  const T unR = uR * n[0] + vR * n[1];
-  const T hm = T(0.5) * (hL + hR);
-  const T hL_sqrt = sqrt_rn(hL);
-  const T hR_sqrt = sqrt_rn(hR);
-  const T um = div_rn((unL * hL_sqrt + unR * hR_sqrt), (hL_sqrt + hR_sqrt + es));
-  const T smax = fabs(um) + fabs(sqrt_rn(g * hm));
-  const T termL = div_rn((n[0] * qL[1] + n[1] * qL[2]), sq(qL[0]));
-  const T termR = div_rn((n[0] * qR[1] + n[1] * qR[2]), sq(qR[0]));
-  const T hsqrt_un = hL_sqrt * unL + hR_sqrt * unR + es;
   const T two_pow_1p5 = T(2.) * sqrt(T(2.));
-  T dL[3], dR[3];
-  dL[0] = div_rn(-fabs(hsqrt_un), (T(2.) * hL_sqrt * sq(hL_sqrt + hR_sqrt))) +
-          div_rn((div_rn(T(0.5) * unL, hL_sqrt) - hL_sqrt * termL) * hsqrt_un, ((hL_sqrt + hR_sqrt) * fabs(hsqrt_un))) +
-          div_rn(g, (two_pow_1p5 * sqrt_rn(g * (hL + hR))));
-  dL[1] = div_rn(n[0] * hsqrt_un, (hL_sqrt * (hL_sqrt + hR_sqrt) * fabs(hsqrt_un)));
-  dL[2] = div_rn(n[1] * hsqrt_un, (hL_sqrt * (hL_sqrt + hR_sqrt) * fabs(hsqrt_un)));
-  dR[0] = div_rn(-fabs(hsqrt_un), (T(2.) * hR_sqrt * sq(hL_sqrt + hR_sqrt))) +
-          div_rn((div_rn(T(0.5) * unR, hR_sqrt) - hR_sqrt * termR) * hsqrt_un, ((hL_sqrt + hR_sqrt) * fabs(hsqrt_un))) +
-          div_rn(g, (two_pow_1p5 * sqrt_rn(g * (hL + hR))));
-  dR[1] = div_rn(n[0] * hsqrt_un, (hR_sqrt * (hL_sqrt + hR_sqrt) * fabs(hsqrt_un)));
-  dR[2] = div_rn(n[1] * hsqrt_un, (hR_sqrt * (hL_sqrt + hR_sqrt) * fabs(hsqrt_un)));
-  JL[0] = -T(0.5) * dL[0] * (qR[0] - qL[0]) + T(0.5) * (n[0] * uL + n[1] * vL - qL[0] * termL) + T(0.5) * smax;
-  JL[1] = T(0.5) * n[0] - T(0.5) * dL[1] * (qR[0] - qL[0]);
-  JL[2] = T(0.5) * n[1] - T(0.5) * dL[2] * (qR[0] - qL[0]);
-  JL[3] = T(0.5) * (g * n[0] * qL[0] - qL[1] * termL) - T(0.5) * dL[0] * (qR[1] - qL[1]);
-  JL[4] = n[0] * uL + T(0.5) * n[1] * vL + T(0.5) * smax - T(0.5) * dL[1] * (qR[1] - qL[1]);
-  JL[5] = T(0.5) * n[1] * uL - T(0.5) * dL[2] * (qR[1] - qL[1]);
-  JL[6] = T(0.5) * (g * n[1] * qL[0] - qL[2] * termL) - T(0.5) * dL[0] * (qR[2] - qL[2]);
-  JL[7] = T(0.5) * n[0] * vL - T(0.5) * dL[1] * (qR[2] - qL[2]);
-  JL[8] = n[1] * vL + T(0.5) * n[0] * uL + T(0.5) * smax - T(0.5) * dL[2] * (qR[2] - qL[2]);
-  JR[0] = -T(0.5) * dR[0] * (qR[0] - qL[0]) + T(0.5) * (n[0] * uR + n[1] * vR - qR[0] * termR) - T(0.5) * smax;
-  JR[1] = T(0.5) * n[0] - T(0.5) * dR[1] * (qR[0] - qL[0]);
-  JR[2] = T(0.5) * n[1] - T(0.5) * dR[2] * (qR[0] - qL[0]);
-  JR[3] = T(0.5) * (g * n[0] * qR[0] - qR[1] * termR) - T(0.5) * dR[0] * (qR[1] - qL[1]);
-  JR[4] = n[0] * uR + T(0.5) * n[1] * vR - T(0.5) * smax - T(0.5) * dR[1] * (qR[1] - qL[1]);
-  JR[5] = T(0.5) * n[1] * uR - T(0.5) * dR[2] * (qR[1] - qL[1]);
-  JR[6] = T(0.5) * (g * n[1] * qR[0] - qR[2] * termR) - T(0.5) * dR[0] * (qR[2] - qL[2]);
-  JR[7] = T(0.5) * n[0] * vR - T(0.5) * dR[1] * (qR[2] - qL[2]);
-  JR[8] = n[1] * vR + T(0.5) * n[0] * uR - T(0.5) * smax - T(0.5) * dR[2] * (qR[2] - qL[2]);
+  const T hL = qL[0], hR = qR[0];
+  const T qnL = ax == 0 ? qL[1] : qL[2], qtL = ax == 0 ? qL[2] : qL[1];
+  const T qnR = ax == 0 ? qR[1] : qR[2], qtR = ax == 0 ? qR[2] : qR[1];
+  T unL, utL, unR, utR;
+  if constexpr (sizeof(T) == 8) {
+    const Quot2 a = div2_rn(qnL, qtL, hL + es), b = div2_rn(qnR, qtR, hR + es);
+    unL = a.q0, utL = a.q1, unR = b.q0, utR = b.q1;
+  } else {
+    unL = div_rn(qnL, hL + es), utL = div_rn(qtL, hL + es);
+    unR = div_rn(qnR, hR + es), utR = div_rn(qtR, hR + es);
+  }
+  const T sL = sqrt_rn(hL), sR = sqrt_rn(hR), sum = sL + sR, hsum = hL + hR;
+  T num = unL * sL + unR * sR;
+  if (not_finite(utL) || not_finite(utR)) num = (utL - utL) + (utR - utR);  // NaN
+  const T um = div_rn(num, sum + es);
+  T smax = fabs(um) + fabs(sqrt_rn(g * half_of(hsum)));
+  const T hu = num + es, ahu = fabs(hu);
+  // this side
+  const T h = side == 0 ? hL : hR, s = side == 0 ? sL : sR, un = side == 0 ? unL : unR, ut = side == 0 ? utL : utR;
+  const T qn = side == 0 ? qnL : qnR, qt = side == 0 ? qtL : qtR;
+  const T term = div_rn(qn, sq(h));
+  const T d0 = half_of(div_rn(-ahu, s * sq(sum))) +
+               div_rn((div_rn(half_of(un), s) - s * term) * hu, sum * ahu) +
+               div_rn(g, two_pow_1p5 * sqrt_rn(g * hsum));
+  const T den = s * sum * ahu, dn = div_rn(hu, den);
+  T dt = T(0.);
+  if (not_finite(dn)) dt = div_rn(dt * hu, den);
+  const T dh = hR - hL, dqn = qnR - qnL, dqt = qtR - qtL;
+  if (side != 0) smax = -smax;
+  const T J0n = half_of(T(1.) - dn * dh);
+  const T Jn0 = half_of((g * h - qn * term) - d0 * dqn);
+  const T Jnn = fma_p2(-T(0.5), dn * dqn, fma_p2(T(0.5), smax, un));
+  const T Jt0 = half_of(-(qt * term) - d0 * dqt);
+  const T Jtn = half_of(ut - dn * dqt);
+  const T Jtt = not_finite(dt) ? dt : half_of(un + smax);
+  J[0] = half_of(((un - h * term) - d0 * dh) + smax);
+  J[1] = ax == 0 ? J0n : dt;
+  J[2] = ax == 0 ? dt : J0n;
+  J[3] = ax == 0 ? Jn0 : Jt0;
+  J[4] = ax == 0 ? Jnn : Jtt;
+  J[5] = ax == 0 ? dt : Jtn;
+  J[6] = ax == 0 ? Jt0 : Jn0;
+  J[7] = ax == 0 ? Jtn : dt;
+  J[8] = ax == 0 ? Jtt : Jnn;
+}
+template <typename T>
+PDA_HD void swe_flux_jac_ax(T JL[9], T JR[9], const T qL[3], const T qR[3], T g, int ax) {
+  swe_flux_jac_side(JL, 0, qL, qR, g, ax);
+  swe_flux_jac_side(JR, 1, qL, qR, g, ax);
 }
 template <int AXIS, typename T>
 PDA_HD void swe_flux_jac(T JL[9], T JR[9], const T qL[3],
