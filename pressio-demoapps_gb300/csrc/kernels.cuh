@@ -252,8 +252,8 @@ PDA_HD void face_grad_side(int side, T &u, T g[2 * SchemeTraits<SCHEME>::h], con
     g[0] = side == 0 ? T(1) : T(0);
     g[1] = side == 0 ? T(0) : T(1);
   } else if constexpr (SCHEME == Weno3) {
-    if (side == 0) weno3_neg_grad(u, g, q[0], q[1], q[2], q[3], out);
-    else weno3_pos_grad(u, g, q[0], q[1], q[2], q[3], out);
+    if (side == 0) weno3_neg_grad<M>(u, g, q[0], q[1], q[2], q[3], out);
+    else weno3_pos_grad<M>(u, g, q[0], q[1], q[2], q[3], out);
   } else {
     if (side == 0) weno5_neg_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5], out);
     else weno5_pos_grad<M>(u, g, q[0], q[1], q[2], q[3], q[4], q[5], out);
