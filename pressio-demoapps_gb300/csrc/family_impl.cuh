@@ -52,16 +52,32 @@ void faces_s(const Box &b, const Phys &p, const double *U, double *Fo, cudaStrea
       k_struct_faces<FAM, SCHEME, AXIS><<<div_up(nf, 128), 128, 0, s>>>(b, p, U, Fo);
     } else {
       // tiled kernel: lines of the other two axes in grid x, face chunks in grid y
-      // 64 x 2 threads: measured against 128 x 1, 128 x 2 and 32 x 4
-      constexpr int NR = 2, LANES = 64;
-      using Cfg = TileCfg<SCHEME, LANES>;
       long lines = 1;
       for (int a = 0; a < 3; ++a)
         if (a != AXIS) lines *= (long)(b.hi[a] - b.lo[a]);
       const int nfa = b.hi[AXIS] - b.lo[AXIS] + 1;
-      dim3 grid(div_up(lines, NR), div_up(nfa, Cfg::TW));
-      dim3 block(Cfg::LANES, NR);
-      k_faces_tile<FAM, SCHEME, AXIS, NR, LANES><<<grid, block, 0, s>>>(b, p, U, Fo);
+      auto launch = [&](auto nr, auto lanes, auto split) {
+        constexpr int NR = decltype(nr)::value, LANES = decltype(lanes)::value;
+        constexpr bool SPLIT = decltype(split)::value;
+        const dim3 grid(div_up(lines, NR), div_up(nfa, TileCfg<SCHEME, LANES>::TW));
+        k_faces_tile<FAM, SCHEME, AXIS, NR, LANES, SPLIT>
+            <<<grid, dim3(LANES, NR, SPLIT ? F::ndpc : 1), 0, s>>>(b, p, U, Fo);
+      };
+      using I1 = std::integral_constant<int, 1>;
+      using I2 = std::integral_constant<int, 2>;
+      using I4 = std::integral_constant<int, 4>;
+      using I32 = std::integral_constant<int, 32>;
+      using I64 = std::integral_constant<int, 64>;
+      // A pass whose warps with a warp per dof are all resident at once is bound by one block's chain, which those
+      // shorten (velocity, 40^2 / 130^2 WENO3 23.4 -> 16.8 / 29.1 -> 22.6 us, WENO5 31.6 -> 18.4 / 40.8 -> 35.0, 20^3
+      // WENO5 75 -> 43); beyond, where the flux's warp waits for the others' barrier, they cost as much or more (203^2
+      // 39.7 and 39.8, 60.4 and 58.3; 512^2 138 and 155, 239 and 257; 41 x 37 x 43 105 and 119).
+      const int lanes32 = 32 * div_up(nfa, TileCfg<SCHEME, 32>::TW), lanes64 = 64 * div_up(nfa, TileCfg<SCHEME, 64>::TW);
+      if ((long)lanes32 * F::ndpc * lines <= 1024L * device_sms()) launch(I1{}, I32{}, std::true_type{});
+      // 64 x 2 threads (measured against 128 x 1, 128 x 2 and 32 x 4 on full tiles), unless narrower tiles leave fewer
+      // lanes without a face (256^2 52.9 -> 48.9 and 88.7 -> 76.7 us, 64^3 WENO5 661 -> 580)
+      else if (lanes32 < lanes64) launch(I4{}, I32{}, std::false_type{});
+      else launch(I2{}, I64{}, std::false_type{});
     }
     ++*launches;
   }

@@ -37,7 +37,9 @@
 //
 // Block: LANES threads along the face axis x NR lines; a block produces TW
 // faces of each of its NR lines (TW = LANES - 3 for WENO5, LANES - 2 for
-// WENO3).  Loads along y/z are strided gathers of whole 32-40 byte cells, so
+// WENO3).  Small meshes take a warp per dof instead of a loop over the dofs,
+// and two warps form the two states' halves of the flux (SPLIT): a block's
+// chain is then a third as long, at the price of two barriers.  Loads along y/z are strided gathers of whole 32-40 byte cells, so
 // no sector is fetched for nothing.
 #pragma once
 
@@ -83,18 +85,26 @@ template <int LANES_> struct TileCfg<Weno3, LANES_> {
   static constexpr int H = 2, LANES = LANES_, TW = LANES - 2, NCELL = TW + 3, NA = 2;
 };
 
-// shared memory of one tile: the cells of NR lines and their alpha terms
-template <int FAM, int SCHEME, int NR, int LANES> struct FaceTileSmem {
+// shared memory of one tile: the cells of NR lines and their alpha terms; with
+// a warp per dof (SPLIT) also the face states and the two halves of the flux
+template <int FAM, int LANES> struct FaceTileSplit {
+  double u[2][Fam<FAM>::ndpc][LANES];
+  typename Fam<FAM>::Side side[2][LANES];
+};
+struct FaceTileWhole {};
+template <int FAM, int SCHEME, int NR, int LANES, bool SPLIT = false> struct FaceTileSmem {
   using C = TileCfg<SCHEME, LANES>;
   double sU[NR][Fam<FAM>::ndpc][C::NCELL + 1];
   double sA[NR][Fam<FAM>::ndpc][C::NA][LANES];
+  typename std::conditional<SPLIT, FaceTileSplit<FAM, LANES>, FaceTileWhole>::type sp;
 };
 
 // One tile: lines lineGroup*NR .. +NR-1 of the box (the lines run along AXIS,
 // numbered with the first other axis fastest), faces chunk*TW .. +TW-1 of
-// each line.  Called by every thread of a LANES x NR block.
-template <int FAM, int SCHEME, int AXIS, int NR, int LANES>
-__device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &sm, const Box &b, const Phys &p,
+// each line.  Called by every thread of a LANES x NR block; SPLIT: of a LANES x
+// NR x ndpc block, a thread's z its dof.
+template <int FAM, int SCHEME, int AXIS, int NR, int LANES, bool SPLIT = false>
+__device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES, SPLIT> &sm, const Box &b, const Phys &p,
                                           const double *__restrict__ U, double *__restrict__ Fout,
                                           long lineGroup, int chunk) {
   using F = Fam<FAM>;
@@ -105,6 +115,8 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
   auto &sA = sm.sA;
 
   const int tx = threadIdx.x, ty = threadIdx.y;
+  const int dz = SPLIT ? (int)threadIdx.z : 0;  // this thread's first dof, and the step to its next
+  constexpr int DZ = SPLIT ? NDPC : 1;
   const int nb1 = b.hi[A1] - b.lo[A1], nb2 = b.hi[A2] - b.lo[A2];
   const int nf = b.hi[AXIS] - b.lo[AXIS] + 1;
   const long line = lineGroup * NR + ty;
@@ -124,7 +136,8 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
     const int c = map_cell(f0 - H + k, b.n[AXIS], b.mode[AXIS], mir);
     const double *src = U + (base + (long)c * stride[AXIS]) * NDPC;
 #pragma unroll
-    for (int d = 0; d < NDPC; ++d) {
+    for (int e = 0; e < NDPC; e += DZ) {
+      const int d = e + dz;
       double v = __ldg(src + d);
       if (mir && d == b.reflect[AXIS]) v = -v;
       sU[ty][d][k] = v;
@@ -140,7 +153,7 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
                      thirteenOvtwelve = 13. / 12.;
     if (tx + 2 < NCELL) {
 #pragma unroll 1
-      for (int d = 0; d < NDPC; ++d) {
+      for (int d = dz; d < NDPC; d += DZ) {
         const double a = sU[ty][d][tx], m = sU[ty][d][tx + 1], c = sU[ty][d][tx + 2];
         double a3, c3;
         mul_k_all<3, 3>(a, c, a3, c3);
@@ -196,7 +209,7 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
     constexpr double two = 2., oneOvthree = 1. / 3., twoOvthree = 2. / 3.;
     if (tx + 1 < NCELL) {
 #pragma unroll 1
-      for (int d = 0; d < NDPC; ++d) {
+      for (int d = dz; d < NDPC; d += DZ) {
         const double a = sU[ty][d][tx], c = sU[ty][d][tx + 1];
         const double X = a - c;
         double B, e, q;
@@ -222,12 +235,24 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
 
   // ---- phase C: face f = f0 + tx between cells f-1 and f
   const int f = f0 + tx;
-  if (!lineOk || tx >= TW || f > b.hi[AXIS]) return;
+  const bool faceOk = lineOk && tx < TW && f <= b.hi[AXIS];
+  if (!SPLIT && !faceOk) return;
   double uN[NDPC], uP[NDPC];
-  if constexpr (SCHEME == Weno5) {
+  auto put_states = [&](int d, double l, double r) {
+    if constexpr (SPLIT) {
+      sm.sp.u[0][d][tx] = l;
+      sm.sp.u[1][d][tx] = r;
+    } else {
+      set_dof(uN, d, l);
+      set_dof(uP, d, r);
+    }
+  };
+  if (SPLIT && !faceOk) {
+    // (no face; the block's barriers below are for all)
+  } else if constexpr (SCHEME == Weno5) {
     constexpr double oneOvsix = 1. / 6.;
 #pragma unroll 1
-    for (int d = 0; d < NDPC; ++d) {
+    for (int d = dz; d < NDPC; d += DZ) {
       // left cell i = f-1: cells i-2..i+3 = sU[tx .. tx+5]; centers i-1..i+2 = sA[.][tx .. tx+3]
       const double qim2 = sU[ty][d][tx], qim1 = sU[ty][d][tx + 1], qi = sU[ty][d][tx + 2];
       const double qip1 = sU[ty][d][tx + 3], qip2 = sU[ty][d][tx + 4], qip3 = sU[ty][d][tx + 5];
@@ -273,13 +298,12 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
         t[4] = w5_term_call(r1, sp, P2);
         t[5] = w5_term_call(r2, sp, P3);
       }
-      set_dof(uN, d, t[0] + t[1] + t[2]);
-      set_dof(uP, d, t[3] + t[4] + t[5]);
+      put_states(d, t[0] + t[1] + t[2], t[3] + t[4] + t[5]);
     }
   } else {
     // p0 = (-q_{i-1} + 3 q_i) / 2, p1 = (q_i + q_{i+1}) / 2, p2 = (3 q_{i+1} - q_{i+2}) / 2
 #pragma unroll 1
-    for (int d = 0; d < NDPC; ++d) {
+    for (int d = dz; d < NDPC; d += DZ) {
       // left cell i = f-1: cells i-1..i+2 = sU[tx .. tx+3]; pairs i-1, i, i+1 = sA[.][tx .. tx+2]
       const double qim1 = sU[ty][d][tx], qi = sU[ty][d][tx + 1], qip1 = sU[ty][d][tx + 2],
                    qip2 = sU[ty][d][tx + 3];
@@ -302,12 +326,30 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
         t[2] = w3_term_call(r0, sp, P1);
         t[3] = w3_term_call(r1, sp, P2);
       }
-      set_dof(uN, d, t[0] + t[1]);
-      set_dof(uP, d, t[2] + t[3]);
+      put_states(d, t[0] + t[1], t[2] + t[3]);
     }
   }
   double fl[NDPC];
-  F::template flux<AXIS, false, true>(fl, uN, uP, p);
+  if constexpr (SPLIT) {
+    // the flux in two halves, then their combination
+    __syncthreads();
+    if (dz < 2 && faceOk) {
+      double q[NDPC];
+#pragma unroll
+      for (int d = 0; d < NDPC; ++d) q[d] = sm.sp.u[dz][d][tx];
+      F::template flux_side<AXIS>(sm.sp.side[dz][tx], q, p);
+    }
+    __syncthreads();
+    if (dz != 0 || !faceOk) return;
+#pragma unroll
+    for (int d = 0; d < NDPC; ++d) {
+      uN[d] = sm.sp.u[0][d][tx];
+      uP[d] = sm.sp.u[1][d][tx];
+    }
+    F::template flux_combine<AXIS>(fl, uN, uP, sm.sp.side[0][tx], sm.sp.side[1][tx], p);
+  } else {
+    F::template flux<AXIS, false, true>(fl, uN, uP, p);
+  }
   // output layout of k_struct_faces: face axis index fastest within its line
   // ordering [A2][A1][face] for AXIS=0, [k][face][i] for AXIS=1, [face][j][i] for AXIS=2
   const int fi = f - b.lo[AXIS];
@@ -325,21 +367,23 @@ __device__ __forceinline__ void face_tile(FaceTileSmem<FAM, SCHEME, NR, LANES> &
 // cap never forces spills that buy no occupancy.  2D Euler, 1024^2, whole
 // velocity: 0.848 ms with 8 blocks of 128 threads (64 registers), 0.857 with
 // 7 (72), 0.868 with 6 (80), 0.910 with 5.
-template <int FAM, int SCHEME, int NR, int LANES>
+template <int FAM, int SCHEME, int NR, int LANES, bool SPLIT = false>
 struct FaceTileMinBlocks {
   static constexpr int kSmemPerSM = 228 * 1024, kReservedPerBlock = 1024;
+  static constexpr int threads = LANES * NR * (SPLIT ? Fam<FAM>::ndpc : 1);
   static constexpr int bySmem =
-      kSmemPerSM / ((int)sizeof(FaceTileSmem<FAM, SCHEME, NR, LANES>) + kReservedPerBlock);
-  static constexpr int byWarps = 1024 / (LANES * NR);
+      kSmemPerSM / ((int)sizeof(FaceTileSmem<FAM, SCHEME, NR, LANES, SPLIT>) + kReservedPerBlock);
+  static constexpr int byWarps = 1024 / threads;
   static constexpr int value = bySmem < byWarps ? (bySmem > 0 ? bySmem : 1) : byWarps;
 };
 
 // grid: x = line groups of NR lines, y = face chunks of TW faces
-template <int FAM, int SCHEME, int AXIS, int NR, int LANES = 64>
-__global__ void __launch_bounds__(LANES *NR, (FaceTileMinBlocks<FAM, SCHEME, NR, LANES>::value))
+template <int FAM, int SCHEME, int AXIS, int NR, int LANES, bool SPLIT = false>
+__global__ void __launch_bounds__((FaceTileMinBlocks<FAM, SCHEME, NR, LANES, SPLIT>::threads),
+                                  (FaceTileMinBlocks<FAM, SCHEME, NR, LANES, SPLIT>::value))
 k_faces_tile(Box b, Phys p, const double *__restrict__ U, double *__restrict__ Fout) {
-  __shared__ FaceTileSmem<FAM, SCHEME, NR, LANES> sm;
-  face_tile<FAM, SCHEME, AXIS, NR, LANES>(sm, b, p, U, Fout, (long)blockIdx.x, (int)blockIdx.y);
+  __shared__ FaceTileSmem<FAM, SCHEME, NR, LANES, SPLIT> sm;
+  face_tile<FAM, SCHEME, AXIS, NR, LANES, SPLIT>(sm, b, p, U, Fout, (long)blockIdx.x, (int)blockIdx.y);
 }
 
 }  // namespace pda
