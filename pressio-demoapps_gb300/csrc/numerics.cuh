@@ -352,6 +352,13 @@ PDA_HD bool not_finite(double x) {
 #endif
 }
 PDA_HD bool not_finite(float x) { return !(x - x == 0.f); }
+PDA_HD bool is_zero(double x) {
+#if defined(__CUDA_ARCH__)
+  return ((uint32_t)__double2hiint(x) << 1 | (uint32_t)__double2loint(x)) == 0u;
+#else
+  return x == 0.;
+#endif
+}
 // x^3 from x and p = x^2 (see cube)
 template <class M>
 PDA_HD double cube_of(double x, double p) {
@@ -749,6 +756,33 @@ PDA_HD void euler5_flux(double F[5], const double qL[5], const double qR[5],
   for (int d = 0; d < 5; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + mx<IP>(smax, qL[d] - qR[d]));
 }
 
+// RN(sqrt(RN(x^2))): |x| itself where the square neither overflows nor
+// underflows (radix 2: S. Boldo, "Stupid is as stupid does", NSV 2015), checked
+// by the integer pipe's operand window; a zero too.
+template <bool INL = false, bool IP = false>
+PDA_HD double root_of_square(double x) {
+#if defined(__CUDA_ARCH__)
+  if (ip::in_window(x) || is_zero(x)) return fabs(x);
+#endif
+  return sqrt_rn<INL>(sqx<IP>(x));
+}
+// Quotients with a dividend that is zero in whole regions (water at rest),
+// which the integer pipe's division would leave to its far, slow exit
+template <bool INL = false>
+PDA_HD double div_or_zero(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  if (is_zero(a) && ip::in_window(b) && __double2hiint(b) >= 0) return a;
+#endif
+  return div_rn<INL>(a, b);
+}
+template <bool INL = false>
+PDA_HD Quot2 div2_or_zero(double a0, double a1, double b) {
+#if defined(__CUDA_ARCH__)
+  if (is_zero(a0) && is_zero(a1) && ip::in_window(b) && __double2hiint(b) >= 0) return {a0, a1};
+#endif
+  return div2_rn<INL>(a0, a1, b);
+}
+
 // Shallow-water Rusanov flux.  deviation: the reference's std::pow(h, 0.5) is
 // evaluated as sqrt(h) (correctly rounded; glibc pow agrees except in rare
 // near-midpoint cases, a 1-ulp difference).
@@ -758,7 +792,7 @@ PDA_HD void swe_flux(double F[3], const double qL[3], const double qR[3],
   constexpr double half = 1. / 2.;
   constexpr double es = 1.e-30;
   const double hL = qL[0];
-  const Quot2 vl = div2_rn<INL>(qL[1], qL[2], esx<IP>(hL));
+  const Quot2 vl = div2_or_zero<INL>(qL[1], qL[2], esx<IP>(hL));
   const double uL = vl.q0, vL = vl.q1;
   const double unL = AXIS == 0 ? uL : vL;
   const double pL = mx<IP>(mx<IP>(halfx<IP>(gravity), hL), hL);
@@ -767,7 +801,7 @@ PDA_HD void swe_flux(double F[3], const double qL[3], const double qR[3],
   FL[1] = AXIS == 0 ? mx<IP>(FL[0], uL) + pL : mx<IP>(FL[0], uL);
   FL[2] = AXIS == 1 ? mx<IP>(FL[0], vL) + pL : mx<IP>(FL[0], vL);
   const double hR = qR[0];
-  const Quot2 vr = div2_rn<INL>(qR[1], qR[2], esx<IP>(hR));
+  const Quot2 vr = div2_or_zero<INL>(qR[1], qR[2], esx<IP>(hR));
   const double uR = vr.q0, vR = vr.q1;
   const double unR = AXIS == 0 ? uR : vR;
   const double pR = mx<IP>(mx<IP>(halfx<IP>(gravity), hR), hR);
@@ -777,9 +811,9 @@ PDA_HD void swe_flux(double F[3], const double qL[3], const double qR[3],
   FR[2] = AXIS == 1 ? mx<IP>(FR[0], vR) + pR : mx<IP>(FR[0], vR);
   const double hm = halfx<IP>(hL + hR);
   const double sL = sqrt_rn<INL>(hL), sR = sqrt_rn<INL>(hR);
-  const double um = div_rn<INL>((mx<IP>(unL, sL) + mx<IP>(unR, sR)), esx<IP>(sL + sR));
+  const double um = div_or_zero<INL>((mx<IP>(unL, sL) + mx<IP>(unR, sR)), esx<IP>(sL + sR));
   const double sg = sqrt_rn<INL>(mx<IP>(gravity, hm));
-  const double smax = sqrt_rn<INL>(sqx<IP>(um)) + sqrt_rn<INL>(sqx<IP>(sg));
+  const double smax = root_of_square<INL, IP>(um) + root_of_square<INL, IP>(sg);
 #pragma unroll
   for (int d = 0; d < 3; ++d) F[d] = halfx<IP>(FL[d] + FR[d] + mx<IP>(smax, qL[d] - qR[d]));
 }
@@ -903,8 +937,8 @@ PDA_HD void euler5_combine(double F[5], const double qL[5], const double qR[5], 
 PDA_HD void swe_side_ax(FluxSide<3> &o, const double q[3], double gravity, int ax) {
   constexpr double es = 1.e-30;
   const double h = q[0];
-  const double u = div_rn(q[1], (h + es));
-  const double v = div_rn(q[2], (h + es));
+  const Quot2 uv = div2_or_zero(q[1], q[2], h + es);
+  const double u = uv.q0, v = uv.q1;
   const double un = ax == 0 ? u : v;
   const double p = 0.5 * gravity * h * h;
   o.F[0] = h * un;
@@ -923,9 +957,9 @@ PDA_HD void swe_combine(double F[3], const double qL[3], const double qR[3], con
   constexpr double half = 1. / 2.;
   constexpr double es = 1.e-30;
   const double hm = 0.5 * (qL[0] + qR[0]);
-  const double um = div_rn((L.u * L.H + R.u * R.H), (L.H + R.H + es));
+  const double um = div_or_zero((L.u * L.H + R.u * R.H), (L.H + R.H + es));
   const double sg = sqrt_rn(gravity * hm);
-  const double smax = sqrt_rn(um * um) + sqrt_rn(sg * sg);
+  const double smax = root_of_square(um) + root_of_square(sg);
 #pragma unroll
   for (int d = 0; d < 3; ++d) F[d] = half * (L.F[d] + R.F[d] + smax * (qL[d] - qR[d]));
 }
