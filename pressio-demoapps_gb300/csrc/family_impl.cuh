@@ -27,8 +27,11 @@ void rows_velocity_s(const RowTable &ta, const RowTable &tb, const MeshArgs &m, 
                      double *V, const StageArgs &st, cudaStream_t s) {
   const int rows = ta.nrows + tb.nrows;
   if (rows <= 0) return;
-  // rows per block: the fewest blocks that still cover every SM once
-  const int rpb = std::max(1, std::min(VelPar<FAM>::RPB_MAX, div_up(rows, device_sms())));
+  // rows per block: the fewest blocks that still cover every SM once, and then as many rows as their warps hold (an
+  // FP64 instruction costs a scheduler the same with few lanes; 1000 cells in 1D: 10 rows where 7 cover the SMs)
+  constexpr int perRow = VelPar<FAM>::NF * VelPar<FAM>::NDPC;
+  const int cover = std::max(1, std::min(VelPar<FAM>::RPB_MAX, div_up(rows, device_sms())));
+  const int rpb = std::min(VelPar<FAM>::RPB_MAX, std::max(cover, pad_warp(cover * perRow) / perRow));
   const int nbA = div_up(ta.nrows, rpb), nb = nbA + div_up(tb.nrows, rpb);
   k_rows_velocity_par<FAM, SCHEME><<<nb, VelPar<FAM>::THREADS, 0, s>>>(ta, tb, nbA, rpb, m, p, U, V, st);
 }

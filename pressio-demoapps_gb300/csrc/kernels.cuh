@@ -927,7 +927,7 @@ k_rows_vj_nearbd_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ 
 // RPB_MAX) are chosen at launch so that small row sets spread over the SMs.
 template <int FAM> struct VelPar {
   static constexpr int NF = 2 * Fam<FAM>::dim, NDPC = Fam<FAM>::ndpc;
-  static constexpr int RPB_MAX = Fam<FAM>::dim == 3 ? 4 : 8;
+  static constexpr int RPB_MAX = Fam<FAM>::dim == 3 ? 4 : Fam<FAM>::dim == 2 ? 8 : 10;
   static constexpr int SIDE = pad_warp(RPB_MAX * NF * NDPC);
   static constexpr int THREADS = 2 * SIDE;
   static constexpr int PART = pad_warp(RPB_MAX * NF);  // one warp: the block's faces
