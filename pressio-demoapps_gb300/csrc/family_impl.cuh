@@ -28,12 +28,23 @@ void rows_velocity_s(const RowTable &ta, const RowTable &tb, const MeshArgs &m, 
   const int rows = ta.nrows + tb.nrows;
   if (rows <= 0) return;
   // rows per block: the fewest blocks that still cover every SM once, and then as many rows as their warps hold (an
-  // FP64 instruction costs a scheduler the same with few lanes; 1000 cells in 1D: 10 rows where 7 cover the SMs)
-  constexpr int perRow = VelPar<FAM>::NF * VelPar<FAM>::NDPC;
-  const int cover = std::max(1, std::min(VelPar<FAM>::RPB_MAX, div_up(rows, device_sms())));
-  const int rpb = std::min(VelPar<FAM>::RPB_MAX, std::max(cover, pad_warp(cover * perRow) / perRow));
-  const int nbA = div_up(ta.nrows, rpb), nb = nbA + div_up(tb.nrows, rpb);
-  k_rows_velocity_par<FAM, SCHEME><<<nb, VelPar<FAM>::THREADS, 0, s>>>(ta, tb, nbA, rpb, m, p, U, V, st);
+  // FP64 instruction costs a scheduler the same with few lanes).  50 SSP-RK3 steps of 1000 cells in 1D, three runs in
+  // flight: 640 us with the 7 rows that cover the SMs, 529 with 10, 498 with 9 rows that share their faces (chained).
+  using VP = VelPar<FAM>;
+  auto rows_per_block = [](const RowTable &t, int cover) {
+    const int perRow = t.chained ? VP::NDPC : VP::NF * VP::NDPC, extra = t.chained ? 1 : 0;
+    const int most = t.chained ? VP::FACES - 1 : VP::RPB_MAX;
+    cover = std::max(1, std::min(most, cover));
+    return std::min(most, std::max(cover, pad_warp((cover + extra) * perRow) / perRow - extra));
+  };
+  const int cover = div_up(rows, device_sms());
+  const bool haveA = ta.nrows > 0;
+  const int rpbA = rows_per_block(haveA ? ta : tb, cover);
+  const int lanes = pad_warp(((haveA ? ta : tb).chained ? rpbA + 1 : rpbA * VP::NF) * VP::NDPC);  // of a side
+  // the other table's rows in blocks as wide
+  const int rpbB = std::max(1, std::min((int)VP::RPB_MAX, lanes / (VP::NF * VP::NDPC)));
+  const int nbA = div_up(ta.nrows, rpbA), nb = nbA + div_up(tb.nrows, rpbB);
+  k_rows_velocity_par<FAM, SCHEME><<<nb, 2 * lanes, 0, s>>>(ta, tb, nbA, rpbA, rpbB, m, p, U, V, st);
 }
 
 void rows_velocity(int scheme, const RowTable &ta, const RowTable &tb, const MeshArgs &m, const Phys &p,

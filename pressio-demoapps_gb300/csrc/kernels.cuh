@@ -923,15 +923,16 @@ k_rows_vj_nearbd_par(RowTable t, MeshArgs m, Phys p, const double *__restrict__ 
 // velocity-only counterpart of k_rows_vj_nearbd_par): thread (side, row, face, dof) one
 // side of the face value (ghost entries through their recipes), thread (row,
 // face) the face flux, thread (row, k) dof k of V in the order of
-// k_rows_velocity.  Bit-identical to k_rows_velocity.  Rows per block (rpb <=
-// RPB_MAX) are chosen at launch so that small row sets spread over the SMs.
+// k_rows_velocity.  Bit-identical to k_rows_velocity.  Rows per block are
+// chosen at launch so that small row sets spread over the SMs and fill their
+// warps.  In 1D the inner rows of a mesh follow one another, and a block forms
+// each face between its rows once.
 template <int FAM> struct VelPar {
   static constexpr int NF = 2 * Fam<FAM>::dim, NDPC = Fam<FAM>::ndpc;
   static constexpr int RPB_MAX = Fam<FAM>::dim == 3 ? 4 : Fam<FAM>::dim == 2 ? 8 : 10;
-  static constexpr int SIDE = pad_warp(RPB_MAX * NF * NDPC);
-  static constexpr int THREADS = 2 * SIDE;
-  static constexpr int PART = pad_warp(RPB_MAX * NF);  // one warp: the block's faces
-  static_assert(2 * PART <= THREADS, "the two face-state halves fit the block");
+  static constexpr int FACES = RPB_MAX * NF;
+  static constexpr int THREADS = 2 * pad_warp(FACES * NDPC);  // at most; as many as the block's faces need
+  static_assert(FACES <= 32, "a warp covers the block's faces");
 };
 
 template <int FAM> struct VelFace {
@@ -942,23 +943,29 @@ template <int FAM> struct VelFace {
 
 template <int FAM, int SCHEME>
 __global__ void __launch_bounds__(VelPar<FAM>::THREADS)
-k_rows_velocity_par(RowTable ta, RowTable tb, int nbA, int rpb, MeshArgs m, Phys p, const double *__restrict__ U,
-                    double *V, StageArgs st) {
+k_rows_velocity_par(RowTable ta, RowTable tb, int nbA, int rpbA, int rpbB, MeshArgs m, Phys p,
+                    const double *__restrict__ U, double *V, StageArgs st) {
   using F = Fam<FAM>;
   using VP = VelPar<FAM>;
   constexpr int NDPC = F::ndpc, DIM = F::dim, H = SchemeTraits<SCHEME>::h, S = 2 * H + 1, G = 2 * H;
   constexpr int NF = VP::NF;
-  __shared__ VelFace<FAM> fd[VP::RPB_MAX][NF];
-  __shared__ typename F::Side sSide[VP::RPB_MAX][NF][2];  // the two face states' halves of each flux
+  __shared__ VelFace<FAM> fd[VP::FACES];
+  __shared__ typename F::Side sSide[VP::FACES][2];  // the two face states' halves of each flux
   // blocks [0, nbA) take the rows of table ta, the others those of tb
   const bool first = (int)blockIdx.x < nbA;
   const RowTable &t = first ? ta : tb;
+  const int rpb = first ? rpbA : rpbB;
   const int tid = threadIdx.x, e0 = (first ? (int)blockIdx.x : (int)blockIdx.x - nbA) * rpb;
+  const int nr = min(rpb, t.nrows - e0);
+  // the block's faces: row rl's are rl * NF + 2 axis (+ 1: right), or rl and rl + 1 where rows share them
+  const bool chained = DIM == 1 && t.chained;
+  const int faces = chained ? nr + 1 : nr * NF;
   {  // one side of one dof's face value
-    const int side = tid / VP::SIDE, slot = tid % VP::SIDE;
-    const int rl = slot / (NF * NDPC), f = (slot / NDPC) % NF, d = slot % NDPC, ax = f >> 1, fs = f & 1;
-    const int e = e0 + rl;
-    if (slot < rpb * NF * NDPC && e < t.nrows) {
+    const int half = (int)blockDim.x / 2, side = tid / half, slot = tid % half;
+    const int fi = slot / NDPC, d = slot % NDPC;
+    if (fi < faces) {
+      const int rl = chained ? min(fi, nr - 1) : fi / NF, f = chained ? fi - rl : fi % NF, ax = f >> 1, fs = f & 1;
+      const int e = e0 + rl;
       const size_t base = ((size_t)e * DIM + ax) * S;
       double q[G];
 #pragma unroll
@@ -968,7 +975,7 @@ k_rows_velocity_par(RowTable ta, RowTable tb, int nbA, int rpb, MeshArgs m, Phys
                          base + fs + s);
         q[s] = qe[d];
       }
-      (side == 0 ? fd[rl][f].uN : fd[rl][f].uP)[d] = face_value_side<SCHEME>(side, q);
+      (side == 0 ? fd[fi].uN : fd[fi].uP)[d] = face_value_side<SCHEME>(side, q);
     }
   }
   __syncthreads();
@@ -976,31 +983,29 @@ k_rows_velocity_par(RowTable ta, RowTable tb, int nbA, int rpb, MeshArgs m, Phys
   // stage costs its longest per-warp FP64 instruction stream): warps 0 / 1
   // the left / right face state's quantities, then warp 0 their combination
   {
-    const int part = tid / VP::PART, slot = tid % VP::PART;
-    const int rl = slot / NF, f = slot % NF, ax = f >> 1;
-    if (part < 2 && slot < rpb * NF && e0 + rl < t.nrows) {
-      const double *q = part == 0 ? fd[rl][f].uN : fd[rl][f].uP;
-      typename F::Side &so = sSide[rl][f][part];
-      F::flux_side_ax(so, q, p, ax);  // one stream for all axes of the warp
+    const int part = tid / 32, fi = tid % 32, ax = chained ? 0 : (fi % NF) >> 1;
+    if (part < 2 && fi < faces) {
+      const double *q = part == 0 ? fd[fi].uN : fd[fi].uP;
+      F::flux_side_ax(sSide[fi][part], q, p, ax);  // one stream for all axes of the warp
     }
   }
   __syncthreads();
-  if (tid < rpb * NF) {
-    const int rl = tid / NF, f = tid % NF;
-    if (e0 + rl < t.nrows) {
-      VelFace<FAM> &o = fd[rl][f];
-      const typename F::Side &L = sSide[rl][f][0], &R = sSide[rl][f][1];
-      F::template flux_combine<0>(o.fl, o.uN, o.uP, L, R, p);  // the combination does not depend on the axis
-    }
+  if (tid < faces) {
+    VelFace<FAM> &o = fd[tid];
+    const typename F::Side &L = sSide[tid][0], &R = sSide[tid][1];
+    F::template flux_combine<0>(o.fl, o.uN, o.uP, L, R, p);  // the combination does not depend on the axis
   }
   __syncthreads();
-  if (tid < rpb * NDPC) {  // dof k of the row's velocity
-    const int rl = tid / NDPC, k = tid % NDPC;
+  for (int w = tid; w < nr * NDPC; w += blockDim.x) {  // dof k of the row's velocity
+    const int rl = w / NDPC, k = w % NDPC;
     const int e = e0 + rl;
-    if (e < t.nrows) {
+    {
       double vk = 0.;
 #pragma unroll
-      for (int ax = 0; ax < DIM; ++ax) vk += m.hinv[ax] * (fd[rl][2 * ax].fl[k] - fd[rl][2 * ax + 1].fl[k]);
+      for (int ax = 0; ax < DIM; ++ax) {
+        const int fi = chained ? rl : rl * NF + 2 * ax;
+        vk += m.hinv[ax] * (fd[fi].fl[k] - fd[fi + 1].fl[k]);
+      }
       if constexpr (FAM == Swe2d) {
         // swe_2d_prob_class.hpp:983-994
         const int c = t.cell[e];

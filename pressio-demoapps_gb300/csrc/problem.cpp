@@ -504,6 +504,10 @@ void build_stencil(const pda_problem &P, Table &T, const std::vector<int32_t> &r
       }
     }
   }
+  // (rows with ghosts keep their own faces)
+  T.chained = D == 1 && !allowGhost;
+  for (size_t e = 0; T.chained && e + 1 < rowList.size(); ++e)
+    T.chained = std::equal(&T.src[e * S + 1], &T.src[e * S + 1] + (S - 1), &T.src[(e + 1) * S]);
 }
 
 // ------------------------------------------------------------ CSR pattern

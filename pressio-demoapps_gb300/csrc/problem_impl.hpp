@@ -63,6 +63,7 @@ struct Table {
   DevBuf<uint8_t> d_flip, d_flip1;
   DevBuf<double> d_jfac, d_gsx, d_gsy, d_gsx1, d_gsy1;
   RowTable t{};
+  bool chained = false;
   bool dirty = true;
   int hostRows() const { return (int)rows.size(); }
   // copy the host tables to the device if they changed since the last copy
@@ -86,6 +87,7 @@ struct Table {
     d_gsx1.upload(gsx1);
     d_gsy1.upload(gsy1);
     t.nrows = (int)rows.size();
+    t.chained = chained;
     t.rows = d_rows.p;
     t.cell = d_cell.p;
     t.src = d_src.p;

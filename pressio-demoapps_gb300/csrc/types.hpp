@@ -33,6 +33,7 @@ struct RowTable {
   const double *gsy1;
   const int *jpos1;        // [nrows][dim][3] block offset for existing neighbours, -1 = none
   const double *jfac;      // [nrows][dim][ndpc] ghost-to-cell derivative factors
+  bool chained;            // 1D: each row's right face is the next row's left one, cell for cell
 };
 
 // Ghost state from the source cell, dof by dof: op 0 copy, 1 negate,
