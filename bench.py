@@ -38,14 +38,14 @@ BYTES_PER_CELL = 16 * NDPC  # read U once + write V once (FP64)
 # + 10 divisions + 3 square roots; two faces per cell plus the 24-flop
 # balance; a division or square root counts as one operation).
 # DRAM bytes (read + write) per cell of one face launch, measured by ncu on
-# k_faces_tile at 2048^2 (x-axis launch: 135.3 MB read + 96.3 MB written);
+# k_faces_tile at 2048^2 (x-axis launch: 136.6 MB read + 108.4 MB written);
 # traffic grows in proportion to the cells, so it scales to other sizes
-FACE_TRAFFIC_BYTES_PER_CELL = (135.32e6 + 96.27e6) / 2048 ** 2
+FACE_TRAFFIC_BYTES_PER_CELL = (136.64e6 + 108.38e6) / 2048 ** 2
 # FP64 instructions the face kernel executes per face (ncu thread-instruction
-# counters dadd + dmul + dfma of the same capture, 270.7 per face): the work
+# counters dadd + dmul + dfma of the same capture, 166.4 per face): the work
 # the FP64 pipe actually does, after the divisions, square roots and
-# products by constants moved to the integer pipe
-FP64_INST_PER_FACE = 270.7
+# products moved to the integer pipe
+FP64_INST_PER_FACE = 166.4
 FLOPS_PER_CELL = 2 * (4 * 2 * (71 + 4) + 65 + 10 + 3) + 24
 L2_FLUSH_BYTES = 256 << 20
 
@@ -953,7 +953,7 @@ def main():
                               "peak_source": "measured DFMA probe (pda_measure_fp64_peak)",
                               "note": "algorithmic FP64 ops (add/mul/div/sqrt = 1) per second of the face kernel "
                                       "against the FP64 instruction issue rate; divisions, square roots and "
-                                      "products by constants run on the integer pipe, so frac exceeds 1; "
+                                      "products run on the integer pipe, so frac exceeds 1; "
                                       "pipe_frac is the FP64 pipe's own occupancy",
                               "inst_per_face": FP64_INST_PER_FACE,
                               "pipe_achieved_ginst_per_s": fp64_inst_face_launch / (face_ms * 1e-3) / 1e9,

@@ -1078,7 +1078,8 @@ void stepper_buffers(pda_problem &P, int nr) {
 // Each stage is part of the evaluation that it consumes (StageArgs); the
 // second writes beside its state, whose other cells are still read.  1000
 // cells, 50 steps: 724 -> 664 us with three runs in flight, with separate
-// stage kernels and with this (1D steps are three dependent launches each).
+// stage kernels and with this (1D steps are three dependent launches each; 498
+// with the row kernels of now and several steps per graph).
 void ssprk3_step(pda_problem &P, double *U, double t, double dt) {
   double *a = P.aux.p, *b = P.r[0].p;
   const double tHalf = t + dt / 2., tNext = t + dt;
