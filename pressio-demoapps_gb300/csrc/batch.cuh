@@ -106,10 +106,21 @@ k_batch_balance_stage(BatchArgs a, const double *Us, const double *__restrict__ 
     if (!balance_values<FAM>(b, m, p, Us + bi.uOff, F + bi.fOff[0], F + bi.fOff[1], F + bi.fOff[2], t, v, cell))
       continue;
     const long q0 = bi.uOff + cell * NDPC;
+    double o[NDPC], s0[NDPC], s1[NDPC], w[NDPC];
 #pragma unroll
-    for (int d = 0; d < NDPC; ++d) {
-      const long q = q0 + d;
-      out[q] = kind == 0 ? x[q] + cb * v[d] : ca * out[q] + cb * x[q] + cc * v[d];
+    for (int d = 0; d < NDPC; ++d) s0[d] = x[q0 + d];
+    if (kind == 0) {
+      scaled(w, v, cb);
+#pragma unroll
+      for (int d = 0; d < NDPC; ++d) out[q0 + d] = s0[d] + w[d];
+    } else {
+#pragma unroll
+      for (int d = 0; d < NDPC; ++d) o[d] = out[q0 + d];
+      scaled(s1, o, ca);
+      scaled(o, s0, cb);
+      scaled(w, v, cc);
+#pragma unroll
+      for (int d = 0; d < NDPC; ++d) out[q0 + d] = s1[d] + o[d] + w[d];
     }
   }
 }
