@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdint>
 #include <memory>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -32,6 +33,7 @@
 #include <cuda_runtime.h>
 
 #include "problem_impl.hpp"
+#include "stream_fork.hpp"
 #include "tc_gemm_api.hpp"
 
 namespace pda {
@@ -371,17 +373,17 @@ void forward_backward(pda_ae &A, int B, const AdamCoef *coef, long slot = 0) {
   forward(A, B, true, slot);
   const AdamCoef c0{};
   cudaStream_t ch = A.s;
+  std::optional<StreamFork> side;
   if (coef) {
     if (!A.chain) {
       int least = 0, greatest = 0;
       check(cudaDeviceGetStreamPriorityRange(&least, &greatest), "stream priorities");
       check(cudaStreamCreateWithPriority(&A.chain, cudaStreamNonBlocking, greatest), "stream");
-      for (cudaEvent_t *e : {&A.evFork, &A.evOut, &A.evFirst, &A.evJoin})
-        check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
     }
+    for (cudaEvent_t *e : {&A.evFork, &A.evOut, &A.evFirst, &A.evJoin})
+      if (!*e) check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
     ch = A.chain;
-    check(cudaEventRecord(A.evFork, A.s), "event");
-    check(cudaStreamWaitEvent(ch, A.evFork, 0), "event");
+    side.emplace(A.s, ch, A.evFork, A.evJoin);
   }
   // dW_l = dA_l^T H_in (A = dA_l^T [out x B], B = H_in^T [in x B]): the update, or the stored gradient
   auto input_transpose = [&](int l, cudaStream_t s) {
@@ -431,12 +433,9 @@ void forward_backward(pda_ae &A, int B, const AdamCoef *coef, long slot = 0) {
   }
   if (coef) check(cudaEventRecord(A.evFirst, ch), "event");
   for (int l = 4; l >= 1; --l) weights(l, ch);
-  if (coef) {
-    check(cudaEventRecord(A.evJoin, ch), "event");
-    check(cudaStreamWaitEvent(A.s, A.evFirst, 0), "event");
-  }
+  if (coef) check(cudaStreamWaitEvent(A.s, A.evFirst, 0), "event");
   weights(0, A.s);
-  if (coef) check(cudaStreamWaitEvent(A.s, A.evJoin, 0), "event");
+  if (side) side->join();
 }
 
 // the losses (sum of squares / (B n)) of the steps that took slots 0..steps-1,

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "problem_impl.hpp"
+#include "stream_fork.hpp"
 
 namespace pda {
 
@@ -692,21 +693,12 @@ void check_launch(pda_problem &P, int n = 1) {
   PDA_CUDA(cudaGetLastError());
 }
 
-// the side stream, behind what the problem's stream has been given; its work
-// is joined before the call returns
-cudaStream_t fork_side(pda_problem &P) {
-  if (!P.side) {
-    PDA_CUDA(cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking));
-    PDA_CUDA(cudaEventCreateWithFlags(&P.evFork, cudaEventDisableTiming));
-    PDA_CUDA(cudaEventCreateWithFlags(&P.evJoin, cudaEventDisableTiming));
-  }
-  PDA_CUDA(cudaEventRecord(P.evFork, P.stream));
-  PDA_CUDA(cudaStreamWaitEvent(P.side, P.evFork, 0));
-  return P.side;
-}
-void join_side(pda_problem &P) {
-  PDA_CUDA(cudaEventRecord(P.evJoin, P.side));
-  PDA_CUDA(cudaStreamWaitEvent(P.stream, P.evJoin, 0));
+// work on the side stream beside the problem's (joined before the call returns)
+StreamFork fork_side(pda_problem &P) {
+  if (!P.side) PDA_CUDA(cudaStreamCreateWithFlags(&P.side, cudaStreamNonBlocking));
+  for (cudaEvent_t *e : {&P.evFork, &P.evJoin})
+    if (!*e) PDA_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  return StreamFork(P.stream, P.side, P.evFork, P.evJoin);
 }
 
 // --------------------------------------------------------------- evaluation
@@ -734,10 +726,15 @@ void velocity(pda_problem &P, const double *U, double *V, double t, cudaEvent_t 
       // (measured on 1024^2 Riemann WENO5 with earlier face kernels: 1.302 ms
       // per velocity against 1.319 ms in sequence).  The profiling path (ev)
       // keeps the sequence, one pass at a time.
-      if (P.dim >= 2) P.L->struct_faces(P.scheme, 1, b, P.phys, U, Fb[1], fork_side(P));
-      P.L->struct_faces(P.scheme, 0, b, P.phys, U, Fb[0], P.stream);
-      if (P.dim == 3) P.L->struct_faces(P.scheme, 2, b, P.phys, U, Fb[2], P.stream);
-      if (P.dim >= 2) join_side(P);
+      if (P.dim >= 2) {
+        StreamFork side = fork_side(P);
+        P.L->struct_faces(P.scheme, 1, b, P.phys, U, Fb[1], side.side());
+        P.L->struct_faces(P.scheme, 0, b, P.phys, U, Fb[0], P.stream);
+        if (P.dim == 3) P.L->struct_faces(P.scheme, 2, b, P.phys, U, Fb[2], P.stream);
+        side.join();
+      } else {
+        P.L->struct_faces(P.scheme, 0, b, P.phys, U, Fb[0], P.stream);
+      }
       const double *Fc[3] = {Fb[0], Fb[1], Fb[2]};
       P.L->struct_balance(b, ma, P.phys, U, Fc, V, st, P.stream);
       check_launch(P, P.dim + 1);
@@ -772,18 +769,19 @@ void velocity_and_jacobian(pda_problem &P, const double *U, double *V, double *J
     build_near_table(P, true);
     pattern_to_device(P);
     P.nearT.sync();
+    auto inner = [&] {
+      int nl = 0;
+      P.L->struct_vj(P.scheme, P.jbox, ma, P.phys, U, P.d_rowptr.p, V, J, P.stream, &nl);
+      check_launch(P, nl);
+    };
+    if (P.nearT.t.nrows == 0) return inner();
     // near-boundary rows beside the inner ones (disjoint rows of V and J), on
     // the side stream: their one launch is a chain of latencies
-    const bool near = P.nearT.t.nrows > 0;
-    cudaStream_t ns = near ? fork_side(P) : P.stream;
-    if (near) {
-      P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, ns);
-      check_launch(P);
-    }
-    int nl = 0;
-    P.L->struct_vj(P.scheme, P.jbox, ma, P.phys, U, P.d_rowptr.p, V, J, P.stream, &nl);
-    check_launch(P, nl);
-    if (near) join_side(P);
+    StreamFork side = fork_side(P);
+    P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, side.side());
+    check_launch(P);
+    inner();
+    side.join();
     return;
   }
   build_inner_table(P, true);
@@ -791,22 +789,26 @@ void velocity_and_jacobian(pda_problem &P, const double *U, double *V, double *J
   pattern_to_device(P);
   P.innerT.sync();
   P.nearT.sync();
-  const bool both = P.innerT.t.nrows > 0 && P.nearT.t.nrows > 0;
-  cudaStream_t ns = P.stream;
-  if (both) {
-    // the two row sets are independent (disjoint rows of V and J): fork the
-    // near-boundary rows onto a second stream and join before returning
-    ns = fork_side(P);
-  }
-  if (P.nearT.t.nrows > 0) {
-    P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, ns);
+  auto near = [&](cudaStream_t s) {
+    P.L->rows_vj_nearbd(P.scheme, P.nearT.t, ma, P.phys, U, P.d_rowptr.p, V, J, s);
     check_launch(P);
-  }
-  if (P.innerT.t.nrows > 0) {
+  };
+  auto inner = [&] {
     P.L->rows_vj_inner(P.scheme, P.innerT.t, ma, P.phys, U, P.d_rowptr.p, V, J, P.stream);
     check_launch(P);
+  };
+  if (P.innerT.t.nrows > 0 && P.nearT.t.nrows > 0) {
+    // the two row sets are independent (disjoint rows of V and J): the
+    // near-boundary rows on the side stream
+    StreamFork side = fork_side(P);
+    near(side.side());
+    inner();
+    side.join();
+  } else if (P.nearT.t.nrows > 0) {
+    near(P.stream);
+  } else if (P.innerT.t.nrows > 0) {
+    inner();
   }
-  if (both) join_side(P);
 }
 
 // ------------------------------------------------------------------ create
