@@ -34,6 +34,7 @@
 
 #include <cuda_runtime.h>
 
+#include "csr_rows.hpp"
 #include "numerics.cuh"
 #include "problem_impl.hpp"
 
@@ -58,14 +59,14 @@ k_system(int scheme, long n, const int *__restrict__ rowptr, const int *__restri
     if (scheme == 0) R[r] = y[r] - yn[r] - dt * f[r];
     else R[r] = y[r] - yn[r] - (dt / 2.) * (f[r] + fn[r]);
   }
-  for (int q = rowptr[r] + lane; q < rowptr[r + 1]; q += LPR) {
+  row_batches<1, LPR>(rowptr[r], rowptr[r + 1], lane, [&](unsigned q) {
     double v = c * J[q];
     if (colidx[q] == r) {
       v += 1.;
       dinv[r] = div_rn(1., v);
     }
     J[q] = v;
-  }
+  });
 }
 
 __global__ void k_minus(long n, const double *__restrict__ x, double *__restrict__ y) {
@@ -175,12 +176,12 @@ __device__ __forceinline__ double row_times(const SolveArgs &a, long r, int lane
   constexpr int UN = 9;
   double s = 0.;
   const int end = __ldg(a.rowptr + r + 1);
-  for (int q = __ldg(a.rowptr + r) + lane; q < end; q += UN * LPR) {
+  row_batches<UN, LPR>(__ldg(a.rowptr + r), end, lane, [&](unsigned q) {
     int c[UN];
     double w[UN];
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
-      const bool in = q + u * LPR < end;
+      const bool in = q + u * LPR < (unsigned)end;
       c[u] = in ? __ldg(a.colidx + q + u * LPR) : -1;
       w[u] = in ? __ldg(a.A + q + u * LPR) : 0.;
     }
@@ -190,7 +191,7 @@ __device__ __forceinline__ double row_times(const SolveArgs &a, long r, int lane
 #pragma unroll
     for (int u = 0; u < UN; ++u)
       if (c[u] >= 0) s = fma(w[u], g[u], s);
-  }
+  });
 #pragma unroll
   for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, LPR);
   return s;
