@@ -328,7 +328,9 @@ void struct_vj_axis(const Box &b, const MeshArgs &m, const Phys &p, const double
   constexpr int A1 = AXIS == 0 ? 1 : 0, A2 = AXIS == 2 ? 1 : 2;
   const long lines = (long)(b.hi[A1] - b.lo[A1]) * (b.hi[A2] - b.lo[A2]);
   const int nfa = b.hi[AXIS] - b.lo[AXIS] + 1;
-  dim3 grid((unsigned)lines, (unsigned)div_up(nfa, Cfg::TW));
+  // a line's tiles in grid y, and in z where they are more than y holds (2.03 million faces)
+  const int tiles = div_up(nfa, Cfg::TW), slabs = div_up(tiles, 65535);
+  const dim3 grid((unsigned)lines, (unsigned)div_up(tiles, slabs), (unsigned)slabs);
   k_jtile<FAM, SCHEME, AXIS><<<grid, dim3(Cfg::LANES, Cfg::NDPC), 0, s>>>(b, m, p, U, rowptr, V, J);
 }
 

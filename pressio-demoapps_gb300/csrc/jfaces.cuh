@@ -277,8 +277,8 @@ template <int FAM, int SCHEME, int AXIS> struct EulerJac {
   }
 };
 
-// grid: x = lines of the box along AXIS (first other axis fastest), y = face
-// chunks of TW faces
+// grid: x = lines of the box along AXIS (first other axis fastest), y and z =
+// face chunks of TW faces, y fastest
 template <int FAM, int SCHEME, int AXIS>
 __global__ void __launch_bounds__(JTileCfg<FAM, SCHEME>::THREADS, JTileCfg<FAM, SCHEME>::MINBLOCKS)
 k_jtile(Box b, MeshArgs m, Phys p, const double *__restrict__ U, const int *__restrict__ rowptr,
@@ -296,7 +296,7 @@ k_jtile(Box b, MeshArgs m, Phys p, const double *__restrict__ U, const int *__re
   int c[3];
   c[A1] = b.lo[A1] + (lineOk ? line % nb1 : 0);
   c[A2] = b.lo[A2] + (lineOk ? line / nb1 : 0);
-  const int f0 = b.lo[AXIS] + (int)blockIdx.y * TW;
+  const int f0 = b.lo[AXIS] + (int)(blockIdx.y + gridDim.y * blockIdx.z) * TW;
   const int f = f0 + tx;  // this thread's face, between cells f - 1 and f
   const bool faceOk = lineOk && f <= b.hi[AXIS];
   const bool cellOk = lineOk && tx < TW && f < b.hi[AXIS];  // cell f: faces tx (left), tx + 1 (right)
