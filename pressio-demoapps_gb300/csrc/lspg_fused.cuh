@@ -107,6 +107,21 @@ __device__ __forceinline__ void lspg_tables(LspgTables &t, int K, int from, int 
   }
 }
 
+// Elimination of pivot d = H_jj outside the integer pipe's window (a basis or a
+// state in extreme units), where the products H_rj H_cj would leave the range of
+// their quotient: H_rc -= (s H_rj H_cj) / m with d = m / s, s a power of two.
+// Out of line: no ordinary pivot comes here.  Returns 1 / d.
+static __device__ __noinline__ double lspg_pivot_scaled(double (*H)[LspgTables::KA + 1], int j, int np, double d,
+                                                        const LspgTables &t) {
+  const int ex = (int)(__double_as_longlong(d) >> 52), cut = min(max(ex, 1), 2045);
+  const double s = __longlong_as_double((long long)(2046 - cut) << 52), m = d * s;
+  for (int q = threadIdx.x; q < np; q += blockDim.x) {
+    const int row = t.pi[q], col = t.pl[q];
+    H[row][col] -= H[row][j] * s * H[col][j] / m;
+  }
+  return s / m;
+}
+
 // reduce the group sums in group order, factor, solve, update (the calling
 // block): L D L^T elimination of the matrix [H g; g^T .] augmented by the
 // right-hand side, whose last row becomes D L^-1 g in the trailing updates (no
@@ -137,14 +152,20 @@ __device__ inline void lspg_solve_rt(int K, int nparts, const double *__restrict
 #pragma unroll 1
   for (int j = 0; j < K; ++j) {
     const double d = H[j][j];
+    const int np = (Ka - 1 - j) * (Ka - j) / 2;
     // positive and finite, tested on the bits (no FP64 instruction)
     const long long db = __double_as_longlong(d);
-    if (!(db > 0 && db < 0x7FF0000000000000LL)) {
-      ok = false;
-      break;
+    if (!(db > 0 && ip::in_window(d))) {
+      if (!(db > 0 && db < 0x7FF0000000000000LL)) {
+        ok = false;
+        break;
+      }
+      const double r = lspg_pivot_scaled(H, j, np, d, t);
+      if (lane == j) rd = r;
+      __syncthreads();
+      continue;
     }
     // trailing lower triangle (the augmented row included): H_rc -= (H_rj H_cj) / d, the product beside the reciprocal
-    const int np = (Ka - 1 - j) * (Ka - j) / 2;
     double h = 0., p = 0.;
     if (q0 < np) {
       h = H[row0][col0];
