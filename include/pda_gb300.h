@@ -409,9 +409,11 @@ pda_status pda_lspg_set_jacobian_precision(pda_lspg *rom, int bits);
  * J_R = I - c dt Jf (c = 1 or 1/2) stop before updating once the l2 norm of
  * the correction is below newton_tol (Pressio's default criterion); each
  * correction is BiCGSTAB with a Jacobi preconditioner to a relative residual
- * of linear_tol.  Full meshes only.  info (may be NULL) receives {Newton
- * iterations in total, most in one step, BiCGSTAB iterations in total, worst
- * final relative linear residual}. */
+ * of linear_tol.  Full meshes only.  The call's device buffers (the CSR values
+ * and thirteen vectors) stay with the problem for its next call if they take up
+ * to 256 MiB; larger ones are freed when the call ends.  info (may be NULL)
+ * receives {Newton iterations in total, most in one step, BiCGSTAB iterations
+ * in total, worst final relative linear residual}. */
 pda_status pda_advance_implicit(pda_problem *p, double *d_U, double t0, double dt, int64_t n_steps, int scheme,
                                 double newton_tol, int newton_max_iters, double linear_tol,
                                 int linear_max_iters, double *info);
