@@ -96,41 +96,56 @@ __global__ void k_gather_rows(const bf16 *__restrict__ data, const int64_t *__re
 // The error gradient dA = dH elu'(pre) of a layer (pre = nullptr: a linear
 // layer, dA = dH) as bf16, its transpose dAT [cols x rows], its column sums
 // (the bias gradient, in row order) and, with `b` given, the Adam update of
-// the bias b (moments mb, vb) on the first `realCols` entries.  One block per
-// 32 columns, 32 rows at a time: one launch where the chain of the backward
-// pass had three.
+// the bias b (moments mb, vb) on the first `realCols` entries.  One launch
+// where the chain of the backward pass had three.  One block per 32 columns,
+// since the sums go through the rows in order; what a block takes is latency, so
+// 128 rows are loaded at a time, the next ones while warp 0 adds these up and
+// the other warps write the transpose (all layers' gradients at n = 384, batch
+// 4096: 2.38 ms with 32 rows at a time, 2.00 as three launches).
 __global__ void __launch_bounds__(256)
 k_error_gradient(const float *__restrict__ dH, const float *__restrict__ pre, long rows, long cols,
                  bf16 *__restrict__ dA, bf16 *__restrict__ dAT, float *__restrict__ out, float *__restrict__ b,
                  float *__restrict__ mb, float *__restrict__ vb, long realCols, AdamCoef coef) {
-  __shared__ bf16 t[32][33];
+  constexpr int ROWS = 128, WARPS = 8, PER = ROWS / WARPS;
+  __shared__ bf16 t[ROWS][33];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const long c = (long)blockIdx.x * 32 + x;
-  float s = 0.f;
-  for (long r0 = 0; r0 < rows; r0 += 32) {
+  float d[PER], a[PER];  // this thread's entries of the rows at hand: dH and pre
+  auto load = [&](long r0) {
 #pragma unroll
-    for (int j = y; j < 32; j += 8) {
-      const long r = r0 + j, i = r * cols + c;
-      bf16 v = __float2bfloat16_rn(0.f);
-      if (r < rows && c < cols) {
-        float d = dH[i];
-        if (pre) {
-          const float a = pre[i];
-          d = d * (a > 0.f ? 1.f : expf(a));
-        }
-        v = __float2bfloat16_rn(d);
-        dA[i] = v;
-      }
+    for (int u = 0; u < PER; ++u) {
+      const long r = r0 + y + u * WARPS;
+      const bool in = r < rows && c < cols;
+      d[u] = in ? dH[r * cols + c] : 0.f;
+      a[u] = in && pre ? pre[r * cols + c] : 1.f;
+    }
+  };
+  load(0);
+  float s = 0.f;
+  for (long r0 = 0; r0 < rows; r0 += ROWS) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int j = y + u * WARPS;
+      const long r = r0 + j;
+      const bf16 v = __float2bfloat16_rn(pre ? d[u] * (a[u] > 0.f ? 1.f : expf(a[u])) : d[u]);
+      if (r < rows && c < cols) dA[r * cols + c] = v;
       t[j][x] = v;
     }
     __syncthreads();
+    if (r0 + ROWS < rows) load(r0 + ROWS);
     if (y == 0) {
-      for (int j = 0; j < 32 && r0 + j < rows; ++j) s += __bfloat162float(t[j][x]);
-    }
+      const int n = (int)(rows - r0 < ROWS ? rows - r0 : ROWS);
+#pragma unroll 16
+      for (int j = 0; j < n; ++j) s += __bfloat162float(t[j][x]);
+    } else {
+      for (int j = y - 1; j < 32; j += WARPS - 1) {
+        const long cc = (long)blockIdx.x * 32 + j;
 #pragma unroll
-    for (int j = y; j < 32; j += 8) {
-      const long cc = (long)blockIdx.x * 32 + j, r = r0 + x;
-      if (cc < cols && r < rows) dAT[cc * rows + r] = t[x][j];
+        for (int q = 0; q < ROWS; q += 32) {
+          const long r = r0 + q + x;
+          if (cc < cols && r < rows) dAT[cc * rows + r] = t[q + x][j];
+        }
+      }
     }
     __syncthreads();
   }
