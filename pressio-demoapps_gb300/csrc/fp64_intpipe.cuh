@@ -347,10 +347,6 @@ __device__ __forceinline__ double mul_small_u(double x) {
 __device__ __forceinline__ double mul(double x, double y) {
   return in_window(x, y) ? mul_u(x, y) : mul_call(x, y);
 }
-__device__ __forceinline__ double square(double x) { return in_window(x) ? square_u(x) : mul_call(x, x); }
-__device__ __forceinline__ double mul_const(double x, const double c) {
-  return in_window(x, c) ? mul_const_u(x, c) : mul_call(x, c);
-}
 template <int K>
 __device__ __forceinline__ double mul_small(double x) {
   return in_window(x) ? mul_small_u<K>(x) : mul_call(x, (double)K);

@@ -32,7 +32,7 @@
 // 2,850 FP64 instructions when one thread held it whole (its gradients and
 // Jacobians in 128 registers, 4 warps per scheduler) and takes 1,280 here:
 // terms whose factor is a known zero or one are left out (weno5_side_grad,
-// weno3_side_grad, euler_flux_jac2, EulerJac, the gradient's end components),
+// weno3_side_grad, euler4_flux_jac2, EulerJac, the gradient's end components),
 // exact powers of two join a sum, and the products run on the integer pipe,
 // which the 32 warps per SM of the split by dof can hide.  512^2 WENO5 V + J
 // 3.24 -> 1.87 ms (issue 49 %, FP64 pipe 60 %; a fifth of the stalls wait for

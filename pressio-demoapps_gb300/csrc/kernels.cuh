@@ -80,7 +80,7 @@ template <> struct Fam<Euler2d> {
   static constexpr double jac_scale = 0.5;
   template <int AXIS, class M, class S>
   static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
-    euler_flux_jac2<dim, AXIS, M>(which, fl, set, qL, qR, p.gamma);
+    euler4_flux_jac2<AXIS, M>(which, fl, set, qL, qR, p.gamma);
   }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<4>;
@@ -111,12 +111,8 @@ template <> struct Fam<Euler3d> {
   static PDA_HD void flux_jac_ax(T JL[25], T JR[25], const T qL[5], const T qR[5], const Phys &p, int ax) {
     euler5_flux_jac_ax(JL, JR, qL, qR, (T)p.gamma, ax);
   }
-  // the left (which = 0, with the flux) or right Jacobian times 1 / jac_scale, for the Jacobian tile kernel
+  // the Jacobian tile kernel's Jacobians (EulerJac) are 1 / jac_scale times these
   static constexpr double jac_scale = 0.5;
-  template <int AXIS, class M, class S>
-  static PDA_HD void flux_jac_tile(int which, double *fl, S set, const double *qL, const double *qR, const Phys &p) {
-    euler_flux_jac2<dim, AXIS, M>(which, fl, set, qL, qR, p.gamma);
-  }
   // the flux in two halves (one face state, then the combination); bit-identical to flux
   using Side = FluxSide<5>;
   template <int AXIS>

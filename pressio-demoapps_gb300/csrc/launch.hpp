@@ -58,9 +58,9 @@ const Launchers &launchers_euler3d();
 const Launchers &launchers_swe2d();
 
 // generic device utilities (util.cu)
-void launch_axpby_stage(int kind, double *out, const double *a, const double *b, const double *c,
-                        double ca, double cb, double cc, double cd, const double *d, const double *e,
-                        long n, cudaStream_t s);
+void launch_x_plus_ay(double *out, const double *x, const double *y, double a, long n, cudaStream_t s);
+void launch_rk4_final(double *v, const double *r1, const double *r2, const double *r3, const double *r4, double dt6,
+                      double dt3, long n, cudaStream_t s);
 // FP64 FMA throughput probe: returns FLOP/s measured with CUDA events
 double measure_fp64_fma_rate(int blocks, int threads, int iters, cudaStream_t s);
 // counts = {operand sets, division mismatches, square-root mismatches}

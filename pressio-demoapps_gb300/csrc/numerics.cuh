@@ -108,10 +108,10 @@ PDA_HD float div_rn(float a, float b) { return a / b; }
 template <bool INL = false>
 PDA_HD float sqrt_rn(float x) { return sqrtf(x); }
 
-// The reference's products by small integers (K x), by 1/2 and 1/4, by
-// constants, and its density guard r + 1e-30.  Device code forms the double results on the
-// integer pipe (fp64_intpipe.cuh: the IEEE round-to-nearest values, bit for
-// bit); host code and single precision use the operators.
+// The reference's products by small integers (K x) and by 1/2, products of two
+// variables, and its density guard r + 1e-30.  Device code forms the double
+// results on the integer pipe (fp64_intpipe.cuh: the IEEE round-to-nearest
+// values, bit for bit); host code and single precision use the operators.
 template <int K, typename T>
 PDA_HD T mul_k(T x) {
 #if defined(__CUDA_ARCH__) && !defined(PDA_FP64_PIPE_DIVSQRT)
@@ -125,21 +125,6 @@ PDA_HD T half_of(T x) {
   if constexpr (sizeof(T) == 8) return ip::mul_pow2_neg<1>(x);
 #endif
   return T(1. / 2.) * x;
-}
-template <typename T>
-PDA_HD T quarter_of(T x) {
-#if defined(__CUDA_ARCH__) && !defined(PDA_FP64_PIPE_DIVSQRT)
-  if constexpr (sizeof(T) == 8) return ip::mul_pow2_neg<2>(x);
-#endif
-  return T(1. / 4.) * x;
-}
-// RN(c x) for a positive literal constant c (1/6, 13/12, 2e-6)
-PDA_HD double mul_c(double x, double c) {
-#if defined(__CUDA_ARCH__) && !defined(PDA_FP64_PIPE_DIVSQRT)
-  return ip::mul_const(x, c);
-#else
-  return c * x;
-#endif
 }
 // RN(x y) on the integer pipe, out of line
 PDA_HD double mul_ip_out(double x, double y) {
@@ -156,15 +141,10 @@ PDA_HD double plus_es(double r) {
   return r + 1.e-30;
 #endif
 }
-// Selectable forms of the above: IP = true forms the exact products on the
-// integer pipe (the tile kernels of the residual, where that pays); IP = false
-// keeps the FP64 operations (row, Jacobian and reduced-order kernels, where
-// the extra integer code measured slower).  Both give the same bits.
-template <bool IP, int K, typename T>
-PDA_HD T kx(T x) {
-  if constexpr (IP) return mul_k<K>(x);
-  else return T(K) * x;
-}
+// Selectable forms of the above: IP = true forms them on the integer pipe (the
+// flux in the face tiles, where that pays); IP = false keeps the FP64 operations
+// (row and reduced-order kernels, where the extra integer code measured
+// slower).  Both give the same bits.
 template <bool IP, typename T>
 PDA_HD T halfx(T x) {
   if constexpr (IP) return half_of(x);
@@ -188,19 +168,6 @@ PDA_HD double esx(double r) {
 
 
 template <typename T> PDA_HD T sq(T x) { return x * x; }
-// x^3 for the reference's std::pow(x, 3.) (glibc pow, correctly rounded in
-// all but pathological near-midpoint cases).  Computed with Dekker's exact
-// two-product: x*x = p + e and p*x = c + ce exactly, so x^3 = c + ce + e*x
-// with an error of order 2^-106 before the final rounding; the result is the
-// correctly rounded cube except when x^3 lies within that distance of a
-// rounding midpoint.  Used only on the Jacobian path.
-PDA_HD double cube(double x) {
-  const double p = x * x;
-  const double e = fma(x, x, -p);
-  const double c = p * x;
-  const double ce = fma(p, x, -c);
-  return c + (ce + e * x);
-}
 
 // x / d for a constant d with its reciprocal r = RN(1/d), correctly rounded
 // (Markstein's correction step, P. Markstein, IBM J. Res. Dev. 34(1), 1990:
@@ -216,7 +183,6 @@ PDA_HD double div_const(double x, double d, double r) {
 
 // Single precision, for the approximate (inexact Gauss-Newton) Jacobians of
 // the reduced-order model: no exact-rounding constructions are needed there.
-PDA_HD float cube(float x) { return x * x * x; }
 PDA_HD float div_const(float x, float, float r) { return x * r; }
 
 // k x + c rounded once, for k a power of two.  k x is then exact (for
@@ -225,12 +191,6 @@ PDA_HD float div_const(float x, float, float r) { return x * r; }
 // reference's source, in one FP64 instruction instead of two.
 template <typename T>
 PDA_HD T fma_p2(T k, T x, T c) { return fma(k, x, c); }
-
-// x + k w for a tabulated constant k: a zero k makes the product exact (a
-// signed zero, or NaN for an infinite or NaN w, exactly as RN(k w)), so one
-// rounding; otherwise the two separate roundings of the source
-template <typename T>
-PDA_HD T add_table_prod(T x, T k, T w) { return k == T(0.) ? fma(k, w, x) : x + k * w; }
 
 // The reference's WENO5 stencil expressions (impl/weno5.hpp), evaluated left
 // to right as in its source, with the power-of-two products fused:
@@ -241,20 +201,20 @@ PDA_HD T add_table_prod(T x, T k, T w) { return k == T(0.) ? fma(k, w, x) : x + 
 //   w5_pMidL(a, b, c)  = -a + 5 b + 2 c
 //   w5_pMidR(a, b, c)  = 2 a + 5 b - c
 //   w5_pFarR(a, b, c)  = 11 a - 7 b + 2 c
-template <bool IP = false, typename T>
+template <typename T>
 PDA_HD T w5_curv(T a, T m, T c) { return fma_p2(-T(2.), m, a) + c; }
-template <bool IP = false, typename T>
-PDA_HD T w5_slopeL(T a, T m, T c) { return fma_p2(-T(4.), m, a) + kx<IP, 3>(c); }
-template <bool IP = false, typename T>
-PDA_HD T w5_slopeR(T a, T m, T c) { return fma_p2(-T(4.), m, kx<IP, 3>(a)) + c; }
-template <bool IP = false, typename T>
-PDA_HD T w5_pFarL(T a, T b, T c) { return fma_p2(T(2.), a, -kx<IP, 7>(b)) + kx<IP, 11>(c); }
-template <bool IP = false, typename T>
-PDA_HD T w5_pMidL(T a, T b, T c) { return fma_p2(T(2.), c, -a + kx<IP, 5>(b)); }
-template <bool IP = false, typename T>
-PDA_HD T w5_pMidR(T a, T b, T c) { return fma_p2(T(2.), a, kx<IP, 5>(b)) - c; }
-template <bool IP = false, typename T>
-PDA_HD T w5_pFarR(T a, T b, T c) { return fma_p2(T(2.), c, kx<IP, 11>(a) - kx<IP, 7>(b)); }
+template <typename T>
+PDA_HD T w5_slopeL(T a, T m, T c) { return fma_p2(-T(4.), m, a) + T(3.) * c; }
+template <typename T>
+PDA_HD T w5_slopeR(T a, T m, T c) { return fma_p2(-T(4.), m, T(3.) * a) + c; }
+template <typename T>
+PDA_HD T w5_pFarL(T a, T b, T c) { return fma_p2(T(2.), a, -T(7.) * b) + T(11.) * c; }
+template <typename T>
+PDA_HD T w5_pMidL(T a, T b, T c) { return fma_p2(T(2.), c, -a + T(5.) * b); }
+template <typename T>
+PDA_HD T w5_pMidR(T a, T b, T c) { return fma_p2(T(2.), a, T(5.) * b) - c; }
+template <typename T>
+PDA_HD T w5_pFarR(T a, T b, T c) { return fma_p2(T(2.), c, T(11.) * a - T(7.) * b); }
 
 // ---------------------------------------------------------------------------
 // WENO5, one face i+1/2: uNeg from q_{i-2..i+2}, uPos from q_{i-1..i+3}.
@@ -359,7 +319,12 @@ PDA_HD bool is_zero(double x) {
   return x == 0.;
 #endif
 }
-// x^3 from x and p = x^2 (see cube)
+// x^3 from x and p = RN(x^2) for the reference's std::pow(x, 3.) (glibc pow,
+// correctly rounded in all but pathological near-midpoint cases).  With Dekker's
+// exact two-product, x*x = p + e and p*x = c + ce exactly, so x^3 = c + ce + e*x
+// with an error of order 2^-106 before the final rounding; the result is the
+// correctly rounded cube except when x^3 lies within that distance of a
+// rounding midpoint.  Used only on the Jacobian path.
 template <class M>
 PDA_HD double cube_of(double x, double p) {
   const double e = fma(x, x, -p);
@@ -1221,17 +1186,17 @@ PDA_HD void euler5_flux_jac(T JL[25], T JR[25], const T qL[5],
   euler5_flux_jac_ax(JL, JR, qL, qR, gamma, AXIS);
 }
 
-// The 2D (DIM = 2) or 3D Euler face's Rusanov flux fl and twice its two
-// Jacobians, J2L = 2 dF/dqL and J2R = 2 dF/dqR, for a normal along a fixed
-// axis: euler4/5_flux and euler4/5_flux_jac with the products by the normal's
+// The 2D Euler face's Rusanov flux fl and twice its two Jacobians, J2L = 2
+// dF/dqL and J2R = 2 dF/dqR, for a normal along a fixed axis: euler4_flux and
+// euler4_flux_jac with the products by the normal's
 // zeros and ones left out, what the three have in common formed once, and the
 // factors of 1/2 (exact) joined to a sum or left to the caller, who scales by
 // half as much; every other rounding is theirs.  One call forms one of the
 // two (side 0: J2L and the flux, side 1: J2R), so that two warps share a
 // face's work; set(row, column, x) receives the entries.
-template <int DIM, int AXIS, class M, class S>
-PDA_HD void euler_flux_jac2(int which, double *fl, S set, const double *qL, const double *qR, double gamma) {
-  constexpr int N = DIM + 2, E = DIM + 1;
+template <int AXIS, class M, class S>
+PDA_HD void euler4_flux_jac2(int which, double *fl, S set, const double *qL, const double *qR, double gamma) {
+  constexpr int DIM = 2, N = DIM + 2, E = DIM + 1;
   constexpr double es = 1.e-30;
   const double gm1 = gamma - 1.;
   struct Side {

@@ -1099,16 +1099,16 @@ void rk4_step(pda_problem &P, double *U, double t, double dt) {
   double *aux = P.aux.p;
   const double tHalf = t + dt2, tNext = t + dt;
   velocity(P, U, P.r[0].p, t);
-  launch_axpby_stage(0, aux, U, P.r[0].p, nullptr, 0., dt2, 0., 0., nullptr, nullptr, n, P.stream);
+  launch_x_plus_ay(aux, U, P.r[0].p, dt2, n, P.stream);
   check_launch(P);
   velocity(P, aux, P.r[1].p, tHalf);
-  launch_axpby_stage(0, aux, U, P.r[1].p, nullptr, 0., dt2, 0., 0., nullptr, nullptr, n, P.stream);
+  launch_x_plus_ay(aux, U, P.r[1].p, dt2, n, P.stream);
   check_launch(P);
   velocity(P, aux, P.r[2].p, tHalf);
-  launch_axpby_stage(0, aux, U, P.r[2].p, nullptr, 0., dt, 0., 0., nullptr, nullptr, n, P.stream);
+  launch_x_plus_ay(aux, U, P.r[2].p, dt, n, P.stream);
   check_launch(P);
   velocity(P, aux, P.r[3].p, tNext);
-  launch_axpby_stage(2, U, P.r[0].p, P.r[1].p, P.r[2].p, 0., dt3, 0., dt6, P.r[3].p, nullptr, n, P.stream);
+  launch_rk4_final(U, P.r[0].p, P.r[1].p, P.r[2].p, P.r[3].p, dt6, dt3, n, P.stream);
   check_launch(P);
 }
 

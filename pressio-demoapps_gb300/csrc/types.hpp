@@ -100,8 +100,8 @@ struct LspgFlags {
 };
 
 // What becomes of the velocity v of an evaluation (entry q): stored (kind -1),
-// or the explicit stage that consumes it, with the association of the
-// stand-alone update kernels (util.cu),
+// or the explicit stage that consumes it, with the association of Pressio's
+// ops::update (util.cu),
 //   kind 0: out = x + cb v
 //   kind 1: out = ca y + cb x + cc v
 // so that a stage needs no velocity buffer and no launch of its own.  out is

@@ -7,20 +7,14 @@
 namespace pda {
 namespace {
 
-// Stage updates with the association of Pressio's ops::update on Eigen
+// RK4's stage updates with the association of Pressio's ops::update on Eigen
 // vectors (tests_cpp/pressio/include/pressio/ops/eigen/ops_rank1_update.hpp:
-// 26-46, 67-94, 179-215): v = a*v + b*x + c*y evaluated left to right, and
-// v = b*x + c*y when a == 0.
+// 26-46, 67-94, 179-215), evaluated left to right.  (SSP-RK3's are part of the
+// evaluations' kernels.)
 __global__ void k_x_plus_ay(double *__restrict__ out, const double *__restrict__ x,
                             const double *__restrict__ y, double a, long n) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = x[i] + a * y[i];
-}
-
-__global__ void k_av_bx_cy(double *__restrict__ v, double a, const double *__restrict__ x, double b,
-                           const double *__restrict__ y, double c, long n) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = a * v[i] + b * x[i] + c * y[i];
 }
 
 __global__ void k_rk4_final(double *__restrict__ v, const double *__restrict__ r1,
@@ -111,9 +105,11 @@ __global__ void k_check_divsqrt(int mode, uint64_t seed, long per_thread, unsign
   atomicAdd(bad + 1, ns);
 }
 
-// Operand sets for the comparison of the integer-pipe products by constants
-// (ip::mul_small<K>, ip::mul_pow2_neg<S>, ip::mul_const), of the general
-// product and square (ip::mul, ip::square, counted with the constants) and of
+// Operand sets for the comparison of the integer-pipe products by small integers
+// and powers of two (ip::mul_small<K>, ip::mul_pow2_neg<S>), of the general
+// product (ip::mul), of the unchecked forms that kernels call after a check of
+// their own (ip::mul_u, ip::square_u, ip::mul_const_u; the general products and
+// those by constants are counted together) and of
 // ip::add_1em30 with the FP64 pipe's operations.  mode 0: random mantissas, exponents within 2^-60..2^60;
 // 1: exponents at the edges of the fast paths (subnormal results of the
 // halvings, near-overflow products, the 2^-44 bound of the density guard, the
@@ -160,8 +156,13 @@ __global__ void k_check_products(int mode, uint64_t seed, long per_thread, unsig
     const double y = __longlong_as_double((long long)uy), z = __longlong_as_double((long long)uz);
     nc += !same_bits(z * y, ip::mul(z, y));
     nc += !same_bits(x * z, ip::mul(x, z));
-    nc += !same_bits(z * z, ip::square(z));
-    nc += !same_bits(y * y, ip::square(y));
+    if (ip::in_window(y, z)) {
+      nc += !same_bits(y * z, ip::mul_u(y, z));
+      nc += !same_bits(z * z, ip::square_u(z));
+      nc += !same_bits(y * y, ip::square_u(y));
+    }
+    // as the kernels form the product by a constant
+    auto mul_const = [](double v, const double c) { return ip::in_window(v, c) ? ip::mul_const_u(v, c) : ip::mul_call(v, c); };
     nk += !same_bits(x * 3., ip::mul_small<3>(x));
     nk += !same_bits(x * 5., ip::mul_small<5>(x));
     nk += !same_bits(x * 7., ip::mul_small<7>(x));
@@ -170,13 +171,13 @@ __global__ void k_check_products(int mode, uint64_t seed, long per_thread, unsig
     np += !same_bits(x * 0.5, ip::mul_pow2_neg<1>(x));
     np += !same_bits(x * 0.25, ip::mul_pow2_neg<2>(x));
     ne += !same_bits(x + 1.e-30, ip::add_1em30(x));
-    nc += !same_bits(x * (1. / 6.), ip::mul_const(x, 1. / 6.));
-    nc += !same_bits(x * (13. / 12.), ip::mul_const(x, 13. / 12.));
-    nc += !same_bits(x * (2. * 1e-6), ip::mul_const(x, 2. * 1e-6));
-    nc += !same_bits(x * 0.1, ip::mul_const(x, 0.1));
-    nc += !same_bits(x * 1.4, ip::mul_const(x, 1.4));
-    nc += !same_bits(x * 1e300, ip::mul_const(x, 1e300));
-    nc += !same_bits(x * 1e-300, ip::mul_const(x, 1e-300));
+    nc += !same_bits(x * (1. / 6.), mul_const(x, 1. / 6.));
+    nc += !same_bits(x * (13. / 12.), mul_const(x, 13. / 12.));
+    nc += !same_bits(x * (2. * 1e-6), mul_const(x, 2. * 1e-6));
+    nc += !same_bits(x * 0.1, mul_const(x, 0.1));
+    nc += !same_bits(x * 1.4, mul_const(x, 1.4));
+    nc += !same_bits(x * 1e300, mul_const(x, 1e300));
+    nc += !same_bits(x * 1e-300, mul_const(x, 1e-300));
   }
   atomicAdd(bad, nk);
   atomicAdd(bad + 1, np);
@@ -244,16 +245,14 @@ double measure_fp64_fma_rate(int blocks, int threads, int iters, cudaStream_t s)
   return flops / (ms * 1e-3);
 }
 
-// kind 0: out = a + cb*b
-// kind 1: out = ca*out + cb*a + cc*b
-// kind 2: out = out + cd*a + cb*b + cb*c + cd*d   (RK4 final; cd = dt/6, cb = dt/3)
-void launch_axpby_stage(int kind, double *out, const double *a, const double *b, const double *c,
-                        double ca, double cb, double cc, double cd, const double *d,
-                        const double * /*e*/, long n, cudaStream_t s) {
-  const int g = div_up(n, 256);
-  if (kind == 0) k_x_plus_ay<<<g, 256, 0, s>>>(out, a, b, cb, n);
-  else if (kind == 1) k_av_bx_cy<<<g, 256, 0, s>>>(out, ca, a, cb, b, cc, n);
-  else k_rk4_final<<<g, 256, 0, s>>>(out, a, b, c, d, cd, cb, n);
+// out = x + a*y
+void launch_x_plus_ay(double *out, const double *x, const double *y, double a, long n, cudaStream_t s) {
+  k_x_plus_ay<<<div_up(n, 256), 256, 0, s>>>(out, x, y, a, n);
+}
+// v = v + dt6*r1 + dt3*r2 + dt3*r3 + dt6*r4
+void launch_rk4_final(double *v, const double *r1, const double *r2, const double *r3, const double *r4, double dt6,
+                      double dt3, long n, cudaStream_t s) {
+  k_rk4_final<<<div_up(n, 256), 256, 0, s>>>(v, r1, r2, r3, r4, dt6, dt3, n);
 }
 
 void launch_csr_spmm(long rows, const int *rowptr, const int *colidx, const double *vals, const double *B,
