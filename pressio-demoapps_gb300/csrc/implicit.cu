@@ -171,7 +171,10 @@ __device__ void grid_sums(const double *part, double (&v)[N]) {
   for (int i = 0; i < N; ++i) v[i] = tot[i];
   __syncthreads();
 }
-// row r of A times x, by LPR lanes (all lanes get the sum); a lane's loads go out in batches
+// row r of A times x, by LPR lanes (all lanes get the sum); a lane's loads go out in batches of UN.  Microseconds per
+// BiCGSTAB iteration with UN = 3 / 5 / 9 / 13: rows of 9 entries (3000 1D cells) 20.1 / 20.6 / 22.0 / 22.8, of 36 (64^2;
+// 200^2) 20.5 / 20.9 / 20.3 / 21.0 and 61.7 / 60.5 / 59.6 / 66.3, of 52 (256^2) 191 / 152 / 164 / 142, of 95 (32^3) 189 /
+// 145 / 148 / 140.
 __device__ __forceinline__ double row_times(const SolveArgs &a, long r, int lane, const double *x) {
   constexpr int UN = 9;
   double s = 0.;
@@ -324,16 +327,13 @@ struct Work {
     part.alloc(4 * MAX_BLOCKS);
     arrived.alloc(1);
     info.alloc(1);
-    // every block resident: as many as the SMs hold, no more than the rows fill
-    int dev = 0, sms = 0, occ = 0;
+    // every block resident: one per SM, whose registers 512 threads at 96 each leave no room for a second one, and no
+    // more than the rows fill
+    int dev = 0, sms = 0;
     PDA_CUDA(cudaGetDevice(&dev));
     PDA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PDA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bicgstab, RB, 0));
-    // barriers and sums cost with the blocks, latency without them: one block per SM up to four rounds of
-    // rows, then as many as stay resident
     const long want = (n * LPR + RB - 1) / RB;
-    const long perSm = want <= 4l * sms ? 1 : std::max(occ, 1);
-    blocks = (int)std::max<long>(std::min({want, perSm * sms, (long)MAX_BLOCKS}), 1);
+    blocks = (int)std::max<long>(std::min({want, (long)sms, (long)MAX_BLOCKS}), 1);
   }
 };
 
