@@ -413,8 +413,6 @@ k_struct_faces(Box b, Phys p, const double *__restrict__ U, double *__restrict__
   struct_face<FAM, SCHEME, AXIS>(b, p, U, Fout, (long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// V for every box cell from the face fluxes, in the reference's axis order
-// (x, then y, then z, then the shallow-water Coriolis source).
 // RN(c x[d]) for finite c, on the integer pipe where every x is in its window or
 // zero (uniform flow), checked together.  A balance is bound by the FP64 pipe
 // (24 instructions per 2D Euler cell against 12 so): velocity, 401 x 203 56.9 ->
@@ -437,6 +435,8 @@ __device__ __forceinline__ void scaled(double (&o)[N], const double (&x)[N], dou
   }
 }
 
+// V for every box cell from the face fluxes, in the reference's axis order
+// (x, then y, then z, then the shallow-water Coriolis source).
 template <int FAM>
 __device__ __forceinline__ bool balance_values(const Box &b, const MeshArgs &m, const Phys &p,
                                                const double *__restrict__ U, const double *__restrict__ Fx,

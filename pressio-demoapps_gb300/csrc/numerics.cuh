@@ -51,11 +51,14 @@ template <> struct SchemeTraits<Weno5> { static constexpr int h = 3; };
 // on the integer pipe (fp64_intpipe.cuh): the IEEE round-to-nearest results,
 // bit for bit, without occupying GB300's FP64 pipe (one warp instruction per
 // ~64 cycles per SM sub-partition), which is left to the multiplications and
-// additions.  INL = true expands them in place; otherwise (every kernel of
-// the library) they are calls: inlined, the face kernels outgrew the
-// instruction cache and ran slower.  Host code uses the operators.  Compiling with
-// -DPDA_FP64_PIPE_DIVSQRT selects the FP64-pipe operations on the device too
-// (the same results), for comparison.
+// additions.  INL = true expands them in place (the pivots of the LSPG solve,
+// one division in a serial chain); elsewhere they are calls: inlined, the face
+// kernels outgrew the instruction cache and ran slower.  Host code uses the
+// operators.  Compiling with -DPDA_FP64_PIPE_DIVSQRT selects FP64-pipe divisions,
+// roots, and products that go through the functions of this file on the device
+// too (the same results), for comparison; the groups of products that the tile
+// kernels and the balance check together call ip:: directly and stay on the
+// integer pipe.
 template <bool INL = false>
 PDA_HD double div_rn(double a, double b) {
 #if defined(__CUDA_ARCH__) && !defined(PDA_FP64_PIPE_DIVSQRT)
