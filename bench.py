@@ -708,7 +708,7 @@ def wl_ae_step(c, n=3 * 256 * 256, latent=12, ha=1024, hb=256, batch=128, steps=
     floor_ms = floor_bytes / (hbm * 1e9) * 1e3
     out = {"config": f"autoencoder_adam_step_n{n}_latent12_hidden1024_256_batch128", "parameters": params,
            "hbm_floor_bytes_per_step": floor_bytes, "hbm_floor_ms": floor_ms, "peak_source": src,
-           "note": "host clock around whole epochs of the library's training loop (one loss read back per step)"}
+           "note": "host clock around whole epochs of the library's training loop (the losses read back once per epoch)"}
     for fused in (True, False):
         ae = pda.AutoEncoder(n, latent, ha, hb, seed=1, stream=c.stream)
         ae.set_fused(fused)

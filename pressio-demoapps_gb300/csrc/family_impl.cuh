@@ -189,17 +189,26 @@ int lspg_fused_blocks(int scheme, int innerRows, int nearRows, int K) {
   return div_up(innerRows, rpb) + div_up(nearRows, rpb);
 }
 
-template <typename JT>
-void lspg_fused_prepare_t() {
-  const int bytes = (int)FusedPar<FAM>::kSmemLimit;
-  cudaFuncSetAttribute(k_lspg_fused<FAM, FirstOrder, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_lspg_fused<FAM, Weno3, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_lspg_fused<FAM, Weno5, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+// f(scheme, scalar type of the Jacobian terms, warps side by side) as constants
+template <class Fn>
+void lspg_fused_form(int scheme, bool jac32, bool beside, Fn f) {
+  auto form = [&](auto sc) {
+    if (jac32 && beside) f(sc, float{}, std::true_type{});
+    else if (jac32) f(sc, float{}, std::false_type{});
+    else f(sc, double{}, std::true_type{});
+  };
+  if (scheme == FirstOrder) form(std::integral_constant<int, FirstOrder>{});
+  else if (scheme == Weno3) form(std::integral_constant<int, Weno3>{});
+  else form(std::integral_constant<int, Weno5>{});
 }
 
 void lspg_fused_prepare() {
-  lspg_fused_prepare_t<double>();
-  lspg_fused_prepare_t<float>();
+  for (int scheme : {(int)FirstOrder, (int)Weno3, (int)Weno5})
+    for (int k = 0; k < 3; ++k)
+      lspg_fused_form(scheme, k > 0, k < 2, [](auto sc, auto jt, auto beside) {
+        cudaFuncSetAttribute(k_lspg_fused<FAM, decltype(sc)::value, decltype(jt), decltype(beside)::value>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FusedPar<FAM>::kSmemLimit);
+      });
 }
 
 void lspg_fused(int scheme, const RowTable &ti, const RowTable &tn, const MeshArgs &m, const Phys &p,
@@ -208,21 +217,19 @@ void lspg_fused(int scheme, const RowTable &ti, const RowTable &tn, const MeshAr
   const int nbI = div_up(ti.nrows, rpb);
   const int nb = lspg_fused_blocks(scheme, ti.nrows, tn.nrows, a.K);
   if (nb <= 0) return;
-  constexpr int T = FusedPar<FAM>::THREADS;
   const size_t sm = (size_t)rpb * FusedPar<FAM>::smem_row(2 * (scheme + 1) + 1, a.K);
-  if (a.jac32) {
-    switch (scheme) {
-      case FirstOrder: k_lspg_fused<FAM, FirstOrder, float><<<nb, T, sm, s>>>(ti, tn, rpb, nbI, m, p, a); break;
-      case Weno3: k_lspg_fused<FAM, Weno3, float><<<nb, T, sm, s>>>(ti, tn, rpb, nbI, m, p, a); break;
-      default: k_lspg_fused<FAM, Weno5, float><<<nb, T, sm, s>>>(ti, tn, rpb, nbI, m, p, a); break;
-    }
-    return;
-  }
-  switch (scheme) {
-    case FirstOrder: k_lspg_fused<FAM, FirstOrder, double><<<nb, T, sm, s>>>(ti, tn, rpb, nbI, m, p, a); break;
-    case Weno3: k_lspg_fused<FAM, Weno3, double><<<nb, T, sm, s>>>(ti, tn, rpb, nbI, m, p, a); break;
-    default: k_lspg_fused<FAM, Weno5, double><<<nb, T, sm, s>>>(ti, tn, rpb, nbI, m, p, a); break;
-  }
+  // Two blocks with all warps side by side are resident per SM.  Up to there the shorter chain counts; beyond, with
+  // single-precision terms and few columns, residency: 20 steps of 3276 shallow-water WENO5 rows (410 blocks) K = 2, 8,
+  // 12, 32 913, 1094, 1218, 2995 us side by side and 767, 1013, 1134, 3427 without, of 12,000 1D rows 1785, 2031, 2213,
+  // 4851 and 1418, 1732, 1956, 5464, of 19,660 2D Euler WENO5 rows 3886, 4644, 5365, 15199 and 3355, 4512, 5751, 17486;
+  // 2359 shallow-water rows (295 blocks) 677, 836, 929, 2243 and 678, 844, 928, 2528.  With many columns the products
+  // want the threads, and with double-precision terms the gradients are most of the work.
+  const bool beside = !a.jac32 || a.K > 10 || nb <= 2 * device_sms();
+  lspg_fused_form(scheme, a.jac32, beside, [&](auto sc, auto jt, auto bs) {
+    constexpr bool BESIDE = decltype(bs)::value;
+    k_lspg_fused<FAM, decltype(sc)::value, decltype(jt), BESIDE>
+        <<<nb, FusedPar<FAM>::threads(BESIDE), sm, s>>>(ti, tn, rpb, nbI, m, p, a);
+  });
 }
 
 void rows_vj_nearbd(int scheme, const RowTable &t, const MeshArgs &m, const Phys &p, const double *U,

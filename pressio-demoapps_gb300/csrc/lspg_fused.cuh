@@ -45,8 +45,11 @@ template <int FAM> struct FusedPar {
   static constexpr int RPB_MAX = Fam<FAM>::dim == 3 ? 4 : 8;
   static constexpr int SIDE = pad_warp(RPB_MAX * NF * NDPC);
   static constexpr int PART = pad_warp(RPB_MAX * NF);
-  // phase A's two sides, phase B's four parts, and two warps for the rows' states and histories, side by side
-  static constexpr int THREADS = 2 * SIDE + 4 * PART + 64;
+  // phase A's two sides, phase B's four parts, and two warps for the rows' states and histories: all side by side,
+  // or phase B and these two on phase A's warps
+  static constexpr int threads(bool beside) {
+    return beside ? 2 * SIDE + 4 * PART + 64 : (2 * SIDE > 4 * PART + 64 ? 2 * SIDE : 4 * PART + 64);
+  }
   static_assert(RPB_MAX * NF <= PART && RPB_MAX * NDPC <= 32, "a warp covers the block's faces and rows");
   static constexpr size_t kSmemLimit = 160 * 1024;  // dynamic shared memory per block
   // dynamic shared memory per row: staged D of the row's stencil cells, the
@@ -228,8 +231,11 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // JT: the scalar type of the Jacobian terms (double: the exact Jacobian of
 // the sample-mesh residual; float: an approximate one, on GB300's far wider
 // FP32 units, for an inexact Gauss-Newton step on the same double residual)
-template <int FAM, int SCHEME, typename JT>
-__global__ void __launch_bounds__(FusedPar<FAM>::THREADS)
+// BESIDE: the fluxes and the rows' states on warps beside the face values', a
+// shorter chain for one wave of blocks; without it half as many threads, and so
+// twice as many resident blocks, for grids of several waves
+template <int FAM, int SCHEME, typename JT, bool BESIDE>
+__global__ void __launch_bounds__(FusedPar<FAM>::threads(BESIDE))
 k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p, LspgArgs a) {
   if (!a.first && a.f->converged) return;
   using F = Fam<FAM>;
@@ -247,7 +253,7 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
   __shared__ LspgTables tabs;
   __shared__ typename F::Side sSide[FP::RPB_MAX][NF][2];  // the two face states' halves of the flux
   extern __shared__ double dyn[];
-  constexpr int kHandOver = 2 * FP::SIDE + 4 * FP::PART;
+  constexpr int THREADS = FP::threads(BESIDE), kHandOver = 2 * FP::SIDE + 4 * FP::PART;
   const int tid = threadIdx.x, K = a.K, RD = rpb * NDPC, CB = NDPC * K;  // CB: D doubles per cell
   double *sD = dyn;                                  // [rpb][DIM][S][NDPC][K] staged D of stencil cells
   double *ctb = sD + (size_t)rpb * DIM * S * CB;     // [rpb][NF][NDPC][K]
@@ -262,11 +268,11 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
     const int total = rpb * DIM * npos * chunks;
     // (a round's table entries are loaded before its copies are issued: one wait for the table, not one per copy)
     constexpr int UN = 6;
-    for (int w0 = tid; w0 < total; w0 += UN * FP::THREADS) {
+    for (int w0 = tid; w0 < total; w0 += UN * THREADS) {
       int cell[UN], at[UN];
 #pragma unroll
       for (int u = 0; u < UN; ++u) {
-        const int w = w0 + u * FP::THREADS;
+        const int w = w0 + u * THREADS;
         const int ch = w % chunks, pa = w / chunks, ps = pa % npos, ax = (pa / npos) % DIM, rl = pa / (npos * DIM);
         const int e = e0 + rl;
         at[u] = w < total && e < t.nrows ? ((rl * DIM + ax) * S + ps) * CB + 2 * ch : -1;
@@ -275,12 +281,12 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
       }
 #pragma unroll
       for (int u = 0; u < UN; ++u) {
-        const int ch = (w0 + u * FP::THREADS) % chunks;
+        const int ch = (w0 + u * THREADS) % chunks;
         if (at[u] >= 0) cp_async16(sD + at[u], a.D + (size_t)cell[u] * CB + 2 * ch);
       }
     }
   }
-  // beside phase A: the rows' states and source terms (one warp), the history of their dofs (another), the tables
+  // the rows' states and source terms (one warp), the history of their dofs and the tables (another)
   auto row_state_and_source = [&](int rl) {
     const int e = e0 + rl;
     if (rl >= rpb || e >= t.nrows) return;
@@ -323,7 +329,7 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
     FF &o = fd[rl][f];
     auto hand_over = [&](double v) {
       if (on) (side == 0 ? o.uN : o.uP)[d] = v;
-      bar_arrive<1>(kHandOver);
+      if constexpr (BESIDE) bar_arrive<1>(kHandOver);
     };
     if (inner) {
 #pragma unroll
@@ -353,11 +359,16 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
       }
       hand_over(face_value_side<SCHEME>(side, q));
     }
-  } else if (tid < 2 * FP::SIDE + 4 * FP::PART) {  // phase B: (part, row, face)
-    const int part = (tid - 2 * FP::SIDE) / FP::PART, slot = (tid - 2 * FP::SIDE) % FP::PART;
+  }
+  if constexpr (!BESIDE) __syncthreads();
+  const int tb = BESIDE ? tid - 2 * FP::SIDE : tid;  // this thread's place in phase B and the rows' warps
+  if (tb < 0) {
+    // (phase A's, beside them)
+  } else if (tb < 4 * FP::PART) {  // phase B: (part, row, face)
+    const int part = tb / FP::PART, slot = tb % FP::PART;
     const int rl = slot / NF, f = slot % NF, ax = f >> 1, fs = f & 1;
     const bool on = slot < nrow * NF;
-    bar_wait<1>(kHandOver);
+    if constexpr (BESIDE) bar_wait<1>(kHandOver);
     if (part < 2) {
       // (one stream for all axes of the warp)
       if (on) F::flux_side_ax(sSide[rl][f][part], part == 0 ? fd[rl][f].uN : fd[rl][f].uP, p, ax);
@@ -398,10 +409,10 @@ k_lspg_fused(RowTable ti, RowTable tn, int rpb, int nbInner, MeshArgs m, Phys p,
       if (part == 2) F::flux_jac_ax(o.JN, J2, vN, vP, p, ax);
       else F::flux_jac_ax(J2, o.JP, vN, vP, p, ax);
     }
-  } else if (tid < 2 * FP::SIDE + 4 * FP::PART + 32) {
-    row_state_and_source(tid - 2 * FP::SIDE - 4 * FP::PART);
-  } else {
-    const int rk = tid - 2 * FP::SIDE - 4 * FP::PART - 32;
+  } else if (tb < 4 * FP::PART + 32) {
+    row_state_and_source(tb - 4 * FP::PART);
+  } else if (tb < 4 * FP::PART + 64) {
+    const int rk = tb - 4 * FP::PART - 32;
     if (rk < nrow * NDPC) {
       const int r = t.rows[e0 + rk / NDPC];
       if (rk % NDPC == 0) sRow[rk / NDPC] = r;
