@@ -634,7 +634,8 @@ k_rows_vj_inner(RowTable t, MeshArgs m, Phys p, const double *__restrict__ U,
 // 628 shallow-water WENO5 rows: a block's chain went from 47,000 cycles (18,400
 // in 1a, then 17,500 in 1b with both Jacobians in one warp, 10,000 in phase 2
 // in two warps) to 35,000 (values handed over after 8,200, 1b done at 27,000
-// beside the gradients, 4,500 for phase 2), the call 36.9 -> 20.5 us.  Rows per
+// beside the gradients, 4,500 for phase 2), the call 36.9 -> 20.5 us (18.5 since
+// equal quotients of the Jacobians are merged).  Rows per
 // block fill phase 1a's warps: with one row more than the four of before that
 // case's grid is also within one wave (157 -> 126 blocks; 24.6 us by that and
 // the thread per entry alone).
